@@ -9,27 +9,30 @@
 // Ties of the hard minima are broken in the fixed order same d, d-1, d+1, jump (lowest k for m_q).
 //
 // Mapping, forward: one warp per scanline, lane l holding the K = D/32 consecutive disparities
-// K l .. K l + K - 1; the per-pixel minimum is one REDUX on order-preserving 32-bit keys of the
-// floats (exactly the minimum), the d +- 1 terms stay in the lane except at its edges (one shuffle
-// up, one down). Inputs move in chunks of kFC steps: a row chunk is one contiguous bulk copy, a
-// column chunk one box of a 3D tensor map (TMA), double-buffered on mbarriers with bounded waits;
-// the penalties of a chunk's steps are loaded one chunk ahead, one step per lane. A row scan is a
-// chain of W dependent steps, so everything that does not depend on the path costs is kept off it.
-// Backward: a scanline is held by G lanes of a warp, K = D/G disparities per lane (8 lanes, K = 8
-// at D = 64: the segment buffers fit more lines per SM), minima and sums by butterflies.
+// K l .. K l + K - 1; the per-pixel minimum is one REDUX on the floats, the d +- 1 terms stay in the
+// lane except at its edges (one shuffle up, one down). Inputs move in chunks of kFC positions: a row
+// chunk is one contiguous bulk copy, a column chunk one box of a 3D tensor map (TMA),
+// double-buffered on mbarriers with bounded waits; the penalties are loaded one chunk ahead. A row
+// scan is a chain of W dependent steps, so everything that does not depend on the path costs is
+// kept off it.
 // All four directions run in ONE launch (their blocks side by side, the long row scans first),
 // each writing its own path volume; the soft-argmin kernel adds the four in path order. The
 // backward launch likewise runs the four adjoint scans at once, each writing its own gradient
 // volume and penalty-map gradients, and a last kernel adds them in path order.
 //
-// Backward: per path, scanlines are walked backwards segment by segment; each segment of
-// kSeg pixels is recomputed from the state stored when the forward pass entered it, so no
-// D-deep path volume is kept for the backward (only one state per kSeg pixels). The adjoint
-// routes the gradient of every L_p(d) to C_p(d), to P1(p) or P2(p) through the recorded minimum,
-// and to L_q.
+// Backward: the forward scans record which candidate gave every L_p(d) and where m_q lies (2 bits
+// per voxel and a byte per pixel of each path: a quarter of one volume pass for all four paths), and
+// the adjoint routes the gradient of every L_p(d) to C_p(d), to P1(p) or P2(p) and to L_q by them.
+// Storing path states every 8 pixels and repeating the recurrence in the backward read the cost
+// volume a second time and ran the longer half of the backward's chain: 4 x 1242x375 x 64, scan
+// 1576 -> 772 us, with the recording forward scan at 640 us (645 before, 43.9 -> ~45 instructions a
+// step with the record, ~25 without it).
+// Mapping, backward: a scanline is held by G lanes of a warp, 8 disparities per lane (8 lanes at
+// D = 64), sums by butterflies; the gradient of S is loaded kBwdPF steps ahead. Bound by DRAM:
+// 3.93 GB at 5.1 TB/s at that size.
 //
 // Layouts: cost/sum/grad volumes float [B][H][W][D] (16-byte aligned); maps float [B][H][W];
-// checkpoints float [4 paths][lines][segments][D]. Paths: 0 top->bottom, 1 left->right,
+// records in four slabs of ckpt, one per path. Paths: 0 top->bottom, 1 left->right,
 // 2 bottom->top, 3 right->left.
 #include <cuda_runtime.h>
 
@@ -48,8 +51,8 @@ namespace {
 
 constexpr unsigned kFullMask = 0xFFFFFFFFu;
 constexpr int kK = 8;       // disparities per lane of the soft-argmin kernels
-constexpr int kSeg = 8;     // pixels per recomputed segment (checkpoint interval)
-constexpr int kBwdPF = 2;   // depth of the backward register rings (two interleaved scans per step)
+constexpr int kSeg = 8;     // positions per segment of recorded choices
+constexpr int kBwdPF = 4;   // steps that the backward scans load ahead (divides kSeg)
 constexpr int kWarps = 4;   // warps per block of the scan kernels
 constexpr int kFC = 16;     // steps per staged chunk of the forward scans (a multiple of kSeg)
 // lanes per scanline of the backward scans at D = 64 and D = 32 (any choice gives the same path
@@ -71,18 +74,6 @@ __host__ __device__ inline Geo make_geo(int B, int H, int W, int D, int dir) {
   g.len = horiz ? W : H;
   g.nseg = (g.len + kSeg - 1) / kSeg;
   return g;
-}
-
-// pixel index (b*H + y)*W + x of scan position 0 of `line`, and the pixel stride of one step
-__device__ __forceinline__ void line_origin(const Geo& g, int line, long long& base, long long& step) {
-  if (g.dir == 1 || g.dir == 3) {  // line = b*H + y
-    base = (long long)line * g.W + (g.dir == 3 ? g.W - 1 : 0);
-    step = g.dir == 3 ? -1 : 1;
-  } else {  // line = b*W + x
-    const int b = line / g.W, x = line - b * g.W;
-    base = ((long long)b * g.H + (g.dir == 2 ? g.H - 1 : 0)) * g.W + x;
-    step = g.dir == 2 ? -(long long)g.W : (long long)g.W;
-  }
 }
 
 template <int G>
@@ -126,33 +117,6 @@ __device__ __forceinline__ void storeK(float* p, const float (&v)[K]) {
     reinterpret_cast<float4*>(p)[h] = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
 }
 
-// Neighbours of the lane's disparities d = gl*K + j within the line's group of G lanes.
-template <int G, int K>
-__device__ __forceinline__ void neighbours(const float (&L)[K], int gl, float (&lm)[K], float (&lp)[K]) {
-  const float left = __shfl_up_sync(kFullMask, L[K - 1], 1);
-  const float right = __shfl_down_sync(kFullMask, L[0], 1);
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
-    lm[j] = j > 0 ? L[j - 1] : (gl > 0 ? left : kInf);
-    lp[j] = j < K - 1 ? L[j + 1] : (gl < G - 1 ? right : kInf);
-  }
-}
-
-// One forward step from the previous state Lq into L; returns the new minimum.
-template <int G, int K>
-__device__ __forceinline__ float fstep(const float (&Lq)[K], float (&L)[K], const float (&c)[K], float m, float p1,
-                                       float p2, int gl) {
-  float lm[K], lp[K];
-  neighbours<G, K>(Lq, gl, lm, lp);
-  const float jump = m + p2;
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
-    const float t = fminf(fminf(Lq[j], lm[j] + p1), fminf(lp[j] + p1, jump));
-    L[j] = c[j] + t - m;
-  }
-  return group_min<G>(minK<K>(L));
-}
-
 // Blocks of the four directions side by side in one grid: slot i (direction order[i]) owns blocks
 // [first_block[i], first_block[i + 1]).
 struct Grid4 {
@@ -182,44 +146,97 @@ __device__ __forceinline__ bool locate(const Grid4& q, Line& ln, Geo& g) {
   return true;
 }
 
+// The adjoint needs, per pixel and path, which of the four candidates gave every L_p(d) (2 bits) and
+// the lowest k with L_q(k) = m_q: the forward scans record both, so that the backward scans neither
+// read the cost volume nor repeat the recurrence. Records of a direction live in its checkpoint slab
+// (slab_elems floats), per line and segment of kSeg positions:
+//   codes  32 words (one per forward lane, 2K bits per slot: 32 bits at D = 64, 16 at D = 32)
+//   argmin kSeg bytes
+// Slot t of a segment is the t-th pixel in the order in which the adjoint walks it (against the
+// path): position 7 - t on paths of ascending position, t on descending ones.
+// codes: 0 same d, 1 d-1, 2 d+1, 3 jump (the first of equal candidates).
+template <int K>
+using CodeWord = typename std::conditional<K == 2, uint32_t, uint16_t>::type;
+
+template <int K>
+__host__ __device__ constexpr size_t code_bytes(size_t lines, size_t nseg) {
+  return lines * nseg * 32 * sizeof(CodeWord<K>);
+}
+
 struct FwdArgs {
   const float* cost;
   const float* p1;
   const float* p2;
   float* out[4];   // path volumes, one per direction
-  float* ckpt[4];  // segment entry states, one slab per direction
+  float* rec[4];   // record slabs, one per direction
   Grid4 q;         // one line per warp
 };
 
-// Order-preserving 32-bit key of a (non-NaN) float and back: the unsigned order of the keys is the
-// order of the values, so a REDUX minimum of keys is exactly the minimum.
-__device__ __forceinline__ uint32_t fkey(float f) {
-  const uint32_t b = __float_as_uint(f);
-  return b ^ ((uint32_t)((int32_t)b >> 31) | 0x80000000u);
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
 }
-__device__ __forceinline__ float funkey(uint32_t k) {
-  return __uint_as_float(k ^ ((uint32_t)((int32_t)~k >> 31) | 0x80000000u));
-}
-__device__ __forceinline__ float warp_min(float v) { return funkey(__reduce_min_sync(kFullMask, fkey(v))); }
 
-// One forward step of a warp-held scanline (lane l: d = K l + j), the arithmetic of fstep.
-template <int K>
-__device__ __forceinline__ void fstep_warp(float (&L)[K], const float (&c)[K], float& m, float p1, float p2) {
+// The records of one line being written: the current segment's codes of this lane and argmins.
+struct Rec {
+  uint32_t code = 0, arg[2] = {0, 0};
+};
+
+// One forward step of a warp-held scanline (lane l: d = K l + j) into slot `slot` of r.
+// At K = 2 the edge lanes' shuffles return their own value: lane 0's "d-1" is then its own d+1
+// candidate and lane 31's "d+1" its own d-1 candidate, so no minimum changes and no select is
+// needed; only lane 0's code says 1 for 2, which store_rec puts right.
+template <int K, bool REC>
+__device__ __forceinline__ void fstep_warp(float (&L)[K], const float (&c)[K], float& m, float p1, float p2, Rec& r,
+                                           int slot) {
   const int lane = threadIdx.x & 31;
-  const float left = __shfl_up_sync(kFullMask, L[K - 1], 1);
-  const float right = __shfl_down_sync(kFullMask, L[0], 1);
   const float jump = m + p2;
-  float n[K];
+  if constexpr (REC) {
+    uint32_t arg;  // lowest k with L(k) = m
+    if constexpr (K == 2) {
+      const uint32_t e0 = __ballot_sync(kFullMask, L[0] == m), e1 = __ballot_sync(kFullMask, L[1] == m);
+      const int first = __ffs(e0 | e1) - 1;
+      arg = 2 * first + (((e0 >> (first & 31)) & 1u) ^ 1u);
+    } else {
+      arg = __ffs(__ballot_sync(kFullMask, L[0] == m)) - 1;
+    }
+    r.arg[slot / 4] |= (arg & 0xffu) << (8 * (slot % 4));
+  }
+  float lm[K], lp[K];
+  if constexpr (K == 2) {
+    const float2 a = __fadd2_rn(make_float2(L[0], L[1]), make_float2(p1, p1));
+    lm[0] = __shfl_up_sync(kFullMask, a.y, 1);
+    lp[1] = __shfl_down_sync(kFullMask, a.x, 1);
+    lp[0] = a.y;
+    lm[1] = a.x;
+  } else {
+    const float a = L[0] + p1;
+    const float left = __shfl_up_sync(kFullMask, a, 1), right = __shfl_down_sync(kFullMask, a, 1);
+    lm[0] = lane > 0 ? left : kInf;
+    lp[0] = lane < 31 ? right : kInf;
+  }
+  float t[K];
 #pragma unroll
   for (int j = 0; j < K; ++j) {
-    const float lm = j > 0 ? L[j - 1] : (lane > 0 ? left : kInf);
-    const float lp = j < K - 1 ? L[j + 1] : (lane < 31 ? right : kInf);
-    const float t = fminf(fminf(L[j], lm + p1), fminf(lp + p1, jump));
-    n[j] = c[j] + t - m;
+    t[j] = fminf(fminf(fminf(L[j], lm[j]), lp[j]), jump);
+    if constexpr (REC) {
+      const int sh = 2 * K * slot + 2 * j;
+      const bool q0 = L[j] != t[j], q1 = q0 && lm[j] != t[j], q2 = q1 && lp[j] != t[j];
+      if (q0) r.code += 1u << sh;
+      if (q1) r.code += 1u << sh;
+      if (q2) r.code += 1u << sh;
+    }
   }
-#pragma unroll
-  for (int j = 0; j < K; ++j) L[j] = n[j];
-  m = warp_min(minK<K>(L));
+  if constexpr (K == 2) {
+    const float2 n = __fadd2_rn(__fadd2_rn(make_float2(c[0], c[1]), make_float2(t[0], t[1])), make_float2(-m, -m));
+    L[0] = n.x;
+    L[1] = n.y;
+    m = warp_min(fminf(n.x, n.y));
+  } else {
+    L[0] = c[0] + t[0] - m;
+    m = warp_min(L[0]);
+  }
 }
 
 template <int K>
@@ -229,17 +246,27 @@ __device__ __forceinline__ void ld_lane(const float* p, float (&v)[K]) {
     v[0] = x.x;
     v[1] = x.y;
   } else {
-#pragma unroll
-    for (int j = 0; j < K; ++j) v[j] = p[j];
+    v[0] = p[0];
   }
 }
 template <int K>
 __device__ __forceinline__ void st_lane(float* p, const float (&v)[K]) {
-  if constexpr (K == 2) {
+  if constexpr (K == 2)
     *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
-  } else {
-#pragma unroll
-    for (int j = 0; j < K; ++j) p[j] = v[j];
+  else
+    p[0] = v[0];
+}
+
+// Pixel index of position 0 of a line and the pixel stride of one position (positions ascend with
+// x or y; paths 2 and 3 run through them downwards).
+__device__ __forceinline__ void line_positions(const Geo& g, int line, long long& base, long long& step) {
+  if (g.dir == 1 || g.dir == 3) {  // line = b*H + y
+    base = (long long)line * g.W;
+    step = 1;
+  } else {  // line = b*W + x
+    const int b = line / g.W;
+    base = (long long)b * g.H * g.W + (line - b * g.W);
+    step = g.W;
   }
 }
 
@@ -250,12 +277,13 @@ constexpr size_t fwd_smem_bytes() {
 }
 
 // tm_cost: the cost volume as a 3D tensor map (floats of a row, rows, images), boxes of D x kFC x 1.
-template <int K>
+template <int K, bool REC>
 __global__ void __launch_bounds__(kWarps * 32) k_float_fwd(const __grid_constant__ CUtensorMap tm_cost,
                                                            const FwdArgs a) {
   constexpr int D = 32 * K, C = kFC, NB = 2;
   extern __shared__ __align__(128) float fsm[];
   __shared__ __align__(8) uint64_t bars[kWarps][NB];
+  __shared__ float2 pens[kWarps][NB][C];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) {
     for (int b = 0; b < NB; ++b) sgm::mbar_init(&bars[w][b], 1);
@@ -266,92 +294,125 @@ __global__ void __launch_bounds__(kWarps * 32) k_float_fwd(const __grid_constant
   Geo g;
   if (!locate<32>(a.q, ln, g)) return;  // the whole warp
   long long base, step;
-  line_origin(g, ln.line, base, step);
+  line_positions(g, ln.line, base, step);
   const bool horiz = g.dir == 1 || g.dir == 3;
-  const bool rev = g.dir == 2 || g.dir == 3;  // step j of a chunk at buffer row C - 1 - j
+  const bool rev = g.dir == 2 || g.dir == 3;
   float* box0 = fsm + (size_t)w * NB * C * D;
   const int len = g.len, nch = (len + C - 1) / C;
+  // chunk c holds positions cC .. cC + n - 1 in buffer rows 0 .. n - 1; descending paths take the
+  // chunks, and the positions in them, from the end
+  auto chunk_at = [&](int it) { return rev ? nch - 1 - it : it; };
   auto chunk_n = [&](int c) { return min(C, len - c * C); };
-  auto issue = [&](int c) {  // lane 0
-    const int b = c % NB, n = chunk_n(c);
+  auto issue = [&](int it) {  // lane 0
+    const int b = it % NB, c = chunk_at(it);
     float* dst = box0 + b * C * D;
-    if (horiz) {  // pixels base + (cC + j) step, contiguous; right-to-left: a short chunk at the buffer's end
-      const long long lo = step > 0 ? base + (long long)c * C : base - ((long long)c * C + n - 1);
-      const uint32_t bytes = (uint32_t)(n * D * sizeof(float));
+    if (horiz) {
+      const uint32_t bytes = (uint32_t)(chunk_n(c) * D * sizeof(float));
       sgm::mbar_expect_tx(&bars[w][b], bytes);
-      sgm::bulk_to_smem(dst + (step > 0 ? 0 : (C - n) * D), a.cost + lo * D, bytes, &bars[w][b]);
-    } else {  // column x of image bi: top-to-bottom boxes start at row cC, bottom-to-top ones end at H - cC
+      sgm::bulk_to_smem(dst, a.cost + (base + (long long)c * C) * D, bytes, &bars[w][b]);
+    } else {  // column x of image bi; rows past the image read as zeros
       const int bi = ln.line / g.W, x = ln.line - bi * g.W;
-      const int y0 = g.dir == 0 ? c * C : g.H - C * (c + 1);
       sgm::mbar_expect_tx(&bars[w][b], (uint32_t)(C * D * sizeof(float)));
-      sgm::tma_load_3d(dst, &tm_cost, x * D, y0, bi, &bars[w][b]);
+      sgm::tma_load_3d(dst, &tm_cost, x * D, c * C, bi, &bars[w][b]);
     }
   };
-  // the penalties of step `lane` of chunk c
-  auto pen = [&](int c, float& q1, float& q2) {
-    q1 = q2 = 0.f;
-    if (lane < chunk_n(c)) {
+  // the penalties of position `lane` of the chunk of iteration it
+  auto pen = [&](int it, float2& q) {
+    q = make_float2(0.f, 0.f);
+    const int c = chunk_at(it);
+    if (it < nch && lane < chunk_n(c)) {
       const long long p = base + ((long long)c * C + lane) * step;
-      q1 = __ldg(a.p1 + p);
-      q2 = __ldg(a.p2 + p);
+      q = make_float2(__ldg(a.p1 + p), __ldg(a.p2 + p));
     }
   };
   if (lane == 0) {
     issue(0);
     if (nch > 1) issue(1);
   }
-  float c1, c2, n1 = 0.f, n2 = 0.f;
-  pen(0, c1, c2);
+  float2 pq;
+  pen(0, pq);
   uint32_t phase = 0u;  // bit b: parity of buffer b's next phase
   float L[K], m = 0.f;
-  float* out = a.out[g.dir] + lane * K;
-  float* ck = a.ckpt[g.dir] + (size_t)ln.line * g.nseg * D + lane * K;
-  for (int c = 0; c < nch; ++c) {
-    const int b = c % NB, n = chunk_n(c);
-    pen(c + 1, n1, n2);  // a chunk ahead
-    if (!sgm::mbar_wait_warp(&bars[w][b], (phase >> b) & 1u)) {
-      sgm::scan_give_up_mask(bars[w], phase, (1u << b) | (c + 1 < nch ? 1u << ((c + 1) % NB) : 0u));
-      return;
-    }
-    phase ^= 1u << b;
-    __syncwarp();
-    const float* bx = box0 + b * C * D + lane * K;
-    float cv[C][K];
-#pragma unroll
-    for (int j = 0; j < C; ++j) ld_lane<K>(bx + (rev ? C - 1 - j : j) * D, cv[j]);
-    sgm::fence_proxy_async();  // this lane's reads of the buffer before the copy that refills it
-    __syncwarp();
-    if (lane == 0 && c + 2 < nch) issue(c + 2);
-    float* op = out + (base + (long long)c * C * step) * D;  // step 0 of the chunk
-    const long long od = step * D;
-    auto one = [&](int j) {
-      const float P1 = __shfl_sync(kFullMask, c1, j), P2 = __shfl_sync(kFullMask, c2, j);
-      const int s = c * C + j;
-      if (j % kSeg == 0 && (j > 0 || c > 0)) st_lane<K>(ck + (size_t)(s / kSeg) * D, L);  // state entering
-      if (j == 0 && c == 0) {
-#pragma unroll
-        for (int t = 0; t < K; ++t) L[t] = cv[0][t];
-        m = warp_min(minK<K>(L));
-      } else {
-        fstep_warp<K>(L, cv[j], m, P1, P2);
+  const long long od = step * D;
+  auto* codes = reinterpret_cast<CodeWord<K>*>(a.rec[g.dir]) + (size_t)ln.line * g.nseg * 32 + lane;
+  uint2* args = reinterpret_cast<uint2*>(reinterpret_cast<char*>(a.rec[g.dir]) + code_bytes<K>(g.lines, g.nseg)) +
+                (size_t)ln.line * g.nseg;
+  auto run = [&](auto rev_c, float* out) {
+    constexpr bool REV = decltype(rev_c)::value;
+    for (int it = 0; it < nch; ++it) {
+      const int b = it % NB, c = chunk_at(it), n = chunk_n(c);
+      if (lane < C) pens[w][b][lane] = pq;
+      pen(it + 1, pq);  // a chunk ahead
+      if (!sgm::mbar_wait_warp(&bars[w][b], (phase >> b) & 1u)) {
+        sgm::scan_give_up_mask(bars[w], phase, (1u << b) | (it + 1 < nch ? 1u << ((it + 1) % NB) : 0u));
+        return;
       }
-      st_lane<K>(op + j * od, L);
-    };
-    if (n == C) {
+      phase ^= 1u << b;
+      __syncwarp();
+      const float* bx = box0 + b * C * D + lane * K;
+      float cv[C][K];
 #pragma unroll
-      for (int j = 0; j < C; ++j) one(j);
-    } else {  // the last, short chunk
+      for (int j = 0; j < C; ++j) ld_lane<K>(bx + j * D, cv[j]);
+      sgm::fence_proxy_async();  // this lane's reads of the buffer before the copy that refills it
+      __syncwarp();
+      if (lane == 0 && it + 2 < nch) issue(it + 2);
+      float* op = out + (base + (long long)c * C * step) * D;  // position 0 of the chunk
+      const int first = REV ? len - 1 - c * C : -c * C;        // the path's first pixel, as a row of this chunk
+      Rec r;
+      auto one = [&](int j) {
+        const int slot = REV ? j % kSeg : kSeg - 1 - j % kSeg;
+        if (j == first) {
 #pragma unroll
-      for (int j = 0; j < C; ++j)
-        if (j < n) one(j);
+          for (int t = 0; t < K; ++t) L[t] = cv[j][t];
+          m = warp_min(minK<K>(L));
+        } else {
+          const float2 P = pens[w][b][j];
+          fstep_warp<K, REC>(L, cv[j], m, P.x, P.y, r, slot);
+        }
+        st_lane<K>(op + j * od, L);
+      };
+      auto store_rec = [&](int h) {  // segment h of the chunk
+        if (!REC) return;
+        const int seg = c * (C / kSeg) + h;
+        if (seg < g.nseg) {
+          if (K == 2 && lane == 0) {  // d = 0 has no d-1: its code 1 is the d+1 candidate
+            const uint32_t x = r.code & ~(r.code >> 1) & 0x11111111u;
+            r.code ^= 3u * x;
+          }
+          codes[(size_t)seg * 32] = (CodeWord<K>)r.code;
+          if (lane == 0) args[seg] = make_uint2(r.arg[0], r.arg[1]);
+        }
+        r = Rec();
+      };
+      const bool whole = n == C && (first < 0 || first >= C);
+      if (whole) {
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          const int j = REV ? C - 1 - i : i;
+          const int slot = REV ? j % kSeg : kSeg - 1 - j % kSeg;
+          const float2 P = pens[w][b][j];
+          fstep_warp<K, REC>(L, cv[j], m, P.x, P.y, r, slot);
+          st_lane<K>(op + j * od, L);
+          if (i % kSeg == kSeg - 1) store_rec(j / kSeg);
+        }
+      } else {  // a short chunk, or the one with the path's first pixel
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          const int j = REV ? C - 1 - i : i;
+          if (j < n) one(j);
+          if (i % kSeg == kSeg - 1) store_rec(j / kSeg);
+        }
+      }
     }
-    c1 = n1;
-    c2 = n2;
-  }
+  };
+  if (rev)
+    run(std::true_type{}, a.out[g.dir] + lane * K);
+  else
+    run(std::false_type{}, a.out[g.dir] + lane * K);
 }
 
-// S = ((L0 + L1) + L2) + L3 written over L0; disp = sum_d d softmax(-S/T)
-template <int G>
+// S = ((L0 + L1) + L2) + L3, written over L0 for a backward pass; disp = sum_d d softmax(-S/T)
+template <int G, bool STORE>
 __global__ void __launch_bounds__(256) k_soft_argmin_fwd(float* __restrict__ sum, const float* __restrict__ l1,
                                                          const float* __restrict__ l2, const float* __restrict__ l3,
                                                          float* __restrict__ disp, size_t npix, float inv_t) {
@@ -370,7 +431,7 @@ __global__ void __launch_bounds__(256) k_soft_argmin_fwd(float* __restrict__ sum
   loadK<kK>(l3 + off, d);
 #pragma unroll
   for (int j = 0; j < kK; ++j) S[j] = ((S[j] + b[j]) + c[j]) + d[j];
-  if (live) storeK<kK>(sum + off, S);
+  if (STORE && live) storeK<kK>(sum + off, S);
   const float mn = group_min<G>(minK<kK>(S));
   float z = 0.f, num = 0.f;
 #pragma unroll
@@ -419,197 +480,161 @@ __global__ void __launch_bounds__(256) k_soft_argmin_bwd(const float* __restrict
 }
 
 struct BwdArgs {
-  const float* cost;
-  const float* p1;
-  const float* p2;
   const float* gsum;
-  const float* ckpt[4];
-  float* gout[4];  // gradient volumes, one per direction (written)
-  float* gp1[4];   // penalty-map gradients, one per direction (written)
+  const float* rec[4];  // the forward scans' records
+  float* gout[4];       // gradient volumes, one per direction (written)
+  float* gp1[4];        // penalty-map gradients, one per direction (written)
   float* gp2[4];
   Grid4 q;
 };
 
-// Shared memory of one line: two buffers of (kSeg + 1) states of D floats (slot 0 = state entering
-// the segment), so the recompute of one segment fills one buffer while the adjoint of the segment
-// after it reads the other. Each state is D/4 float4 in the order (quarter h, lane gl); a lane
-// reads back only what it wrote.
-template <int G, int K>
-constexpr size_t bwd_smem_bytes() {
-  return (size_t)kWarps * (32 / G) * 2 * (kSeg + 1) * G * K * sizeof(float);
+// Codes of the lane's K = 8 disparities over one segment: four words; the two bits of voxel t in slot j.
+template <int FK>
+__device__ __forceinline__ constexpr int code_shift(int t, int j) {
+  return FK == 2 ? 4 * j + 2 * (t & 1) : 16 * (t & 1) + 2 * j;
 }
 
+// Sums over the line's G lanes of 2 kSeg values per lane: afterwards lane gl holds in v[0 ..
+// 2 kSeg / G) the sums of values gl * 2 kSeg / G onwards.
+template <int G>
+__device__ __forceinline__ void reduce_segment(float (&v)[2 * kSeg], int gl) {
+  int n = 2 * kSeg;
+#pragma unroll
+  for (int o = G / 2; o; o >>= 1) {
+    n /= 2;
+    const bool hi = gl & o;
+#pragma unroll
+    for (int i = 0; i < kSeg; ++i)
+      if (i < n) {
+        const float send = hi ? v[i] : v[i + n], keep = hi ? v[i + n] : v[i];
+        v[i] = keep + __shfl_xor_sync(kFullMask, send, o);
+      }
+  }
+}
+
+// Adjoint of the four paths. A line is walked against its path; every step adds the gradient that
+// arrives at L_p from its successor to the one of S, writes it (the gradient of C_p) and routes it to
+// the predecessor by the recorded choices: gv goes to L_q(d), L_q(d-1), L_q(d+1) or to m_q, and
+// subtracting m_q takes the sum of all that did not jump from L_q(argmin).
 template <int G, int K>
-__global__ void __launch_bounds__(kWarps * 32, 3) k_float_bwd(const BwdArgs a) {
-  constexpr int D = G * K, Q = D / 4, kSlots = kSeg + 1;
-  extern __shared__ float4 seg_smem[];
+__global__ void __launch_bounds__(kWarps * 32, 4) k_float_bwd(const BwdArgs a) {
+  static_assert(K == 8, "four words of codes per lane and segment");
+  constexpr int D = G * K, FK = D / 32, PF = kBwdPF;
   Line ln;
   Geo g;
   if (!locate<G>(a.q, ln, g)) return;
-  const int lane = threadIdx.x & 31, gl = lane % G, grp = lane / G;
+  const int lane = threadIdx.x & 31, gl = lane % G;
   long long base, step;
-  line_origin(g, ln.line, base, step);
-  float4* st = seg_smem + (size_t)((threadIdx.x >> 5) * (32 / G) + grp) * 2 * kSlots * Q;
-  auto st_put = [&](int buf, int slot, const float (&v)[K]) {
-#pragma unroll
-    for (int h = 0; h < K / 4; ++h)
-      st[(buf * kSlots + slot) * Q + h * G + gl] = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
-  };
-  auto st_get = [&](int buf, int slot, float (&v)[K]) {
-#pragma unroll
-    for (int h = 0; h < K / 4; ++h) {
-      const float4 x = st[(buf * kSlots + slot) * Q + h * G + gl];
-      v[4 * h] = x.x; v[4 * h + 1] = x.y; v[4 * h + 2] = x.z; v[4 * h + 3] = x.w;
-    }
-  };
-  const float* ck = a.ckpt[ln.dir] + (size_t)ln.line * g.nseg * D + gl * K;
-  float* gout = a.gout[ln.dir];
+  line_positions(g, ln.line, base, step);
+  const bool down = ln.dir < 2;  // paths of ascending position are walked downwards
+  const int len = g.len, nseg = g.nseg;
+  const long long sd = step * D;
+  const float* gs = a.gsum + base * D + gl * K;
+  float* go = a.gout[ln.dir] + base * D + gl * K;
   float* gp1 = a.gp1[ln.dir];
   float* gp2 = a.gp2[ln.dir];
-  float gnext[K];
+  const uint4* codes = reinterpret_cast<const uint4*>(reinterpret_cast<const CodeWord<FK>*>(a.rec[ln.dir]) +
+                                                      (size_t)ln.line * nseg * 32) + gl;
+  const uint2* args = reinterpret_cast<const uint2*>(reinterpret_cast<const char*>(a.rec[ln.dir]) +
+                                                     code_bytes<FK>(g.lines, nseg)) + (size_t)ln.line * nseg;
+  const bool live = ln.live;
+  float gn[K];  // gradient arriving from the successor
 #pragma unroll
-  for (int j = 0; j < K; ++j) gnext[j] = 0.f;
-  float LA[K], LB[K];  // recomputed states of even / odd scan positions (segment starts are even)
-  float m = 0.f;
-  float rc[kBwdPF][K], rp1[kBwdPF], rp2[kBwdPF];  // inputs of the recompute steps
-  float rg[kBwdPF][K], rq1[kBwdPF], rq2[kBwdPF];  // inputs of the adjoint steps
-  auto fetch_r = [&](int j, int s) {
-    const long long p = base + s * step;
-    loadK<K>(a.cost + p * D + gl * K, rc[j]);
-    rp1[j] = __ldg(a.p1 + p);
-    rp2[j] = __ldg(a.p2 + p);
+  for (int t = 0; t < K; ++t) gn[t] = 0.f;
+  float ring[PF][K];
+  auto segment = [&](int si) { return down ? nseg - 1 - si : si; };
+  auto position = [&](int seg, int slot) { return seg * kSeg + (down ? kSeg - 1 - slot : slot); };
+  auto fetch = [&](int r, int si, int slot) {  // gradient of S at a slot; nothing past the line
+    if (si >= nseg) return;
+    const int pos = position(segment(si), slot);
+    if (pos < len) loadK<K>(gs + pos * sd, ring[r]);
   };
-  auto fetch_a = [&](int j, int s) {
-    const long long p = base + s * step;
-    loadK<K>(a.gsum + p * D + gl * K, rg[j]);
-    rq1[j] = __ldg(a.p1 + p);
-    rq2[j] = __ldg(a.p2 + p);
-  };
-  // Phase ph recomputes segment kr = last - ph (while ph <= last) and, interleaved with it step
-  // by step, runs the adjoint backwards through segment kr + 1 (from ph = 1 on) over the states
-  // the previous phase recomputed: two independent dependency chains per step.
-  const int last = g.nseg - 1;
-  for (int ph = 0; ph <= last + 1; ++ph) {
-    const int kr = last - ph, ka = kr + 1;
-    const int r0 = kr * kSeg, nr = kr >= 0 ? min(g.len, r0 + kSeg) - r0 : 0;
-    const int a0 = ka * kSeg, na = ph >= 1 ? min(g.len, a0 + kSeg) - a0 : 0;
-    const int br = kr & 1, ba = ka & 1;
-    if (kr > 0) {
-      loadK<K>(ck + (size_t)kr * D, LB);
-      st_put(br, 0, LB);
-      m = group_min<G>(minK<K>(LB));
+#pragma unroll
+  for (int j = 0; j < PF; ++j) fetch(j, 0, j);
+  uint4 cw = __ldg(codes + (size_t)segment(0) * G);
+  uint2 aw = __ldg(args + segment(0));
+  for (int si = 0; si < nseg; ++si) {
+    const int seg = segment(si);
+    const uint32_t w[4] = {cw.x, cw.y, cw.z, cw.w}, ar[2] = {aw.x, aw.y};
+    if (si + 1 < nseg) {
+      cw = __ldg(codes + (size_t)segment(si + 1) * G);
+      aw = __ldg(args + segment(si + 1));
     }
-#pragma unroll
-    for (int j = 0; j < kBwdPF; ++j) {
-      if (j < nr) fetch_r(j, r0 + j);
-      if (j < na) fetch_a(j, a0 + na - 1 - j);
-    }
-    // one recompute step into slot 1 + i of buffer br (L(r0 + i)); one adjoint step at
-    // s = a0 + na - 1 - i (last pixel first). `at_start`: the step may be the path's first pixel.
-    auto r_step = [&](int jr, int i, int n, auto at_start) {
-      const int s = r0 + i;
-      float(&L)[K] = (jr & 1) ? LB : LA;
-      float(&Lq)[K] = (jr & 1) ? LA : LB;
-      float c[K];
-#pragma unroll
-      for (int t = 0; t < K; ++t) c[t] = rc[jr][t];
-      const float P1 = rp1[jr], P2 = rp2[jr];
-      if (i + kBwdPF < n) fetch_r(jr, s + kBwdPF);
-      if (decltype(at_start)::value && s == 0) {
-#pragma unroll
-        for (int t = 0; t < K; ++t) L[t] = c[t];
-        m = group_min<G>(minK<K>(L));
-      } else {
-        m = fstep<G, K>(Lq, L, c, m, P1, P2, gl);
-      }
-      st_put(br, 1 + i, L);
-    };
-    auto a_step = [&](int jr, int i, int n, auto at_start) {
-      const int s = a0 + na - 1 - i;
-      const long long p = base + s * step;
+    float part[2 * kSeg];  // this lane's share of the P1 and P2 gradients of each slot
+    auto step_at = [&](int j, bool start) {
+      const long long off = position(seg, j) * sd;
       float gv[K];
 #pragma unroll
-      for (int t = 0; t < K; ++t) gv[t] = rg[jr][t] + gnext[t];
-      const float P1 = rq1[jr], P2 = rq2[jr];
-      if (i + kBwdPF < n) fetch_a(jr, s - kBwdPF);
-      if (ln.live) storeK<K>(gout + p * D + gl * K, gv);
-      if (decltype(at_start)::value && s == 0) {  // the first pixel of a path adds nothing to the penalties
-        if (ln.live && gl == 0) {
-          gp1[p] = 0.f;
-          gp2[p] = 0.f;
-        }
-      } else {
-        // previous state L_q = L(s-1): slot (s - a0) (slot 0 = checkpoint when s == a0)
-        float Lq[K];
-        st_get(ba, s - a0, Lq);
-        // m_q and its (lowest) index
-        float mn = Lq[0];
-        int mi = gl * K;
+      for (int t = 0; t < K; t += 2) {
+        const float2 x = __fadd2_rn(make_float2(ring[j % PF][t], ring[j % PF][t + 1]), make_float2(gn[t], gn[t + 1]));
+        gv[t] = x.x;
+        gv[t + 1] = x.y;
+      }
+      fetch(j % PF, j + PF < kSeg ? si : si + 1, (j + PF) % kSeg);
+      if (live) storeK<K>(go + off, gv);
+      part[2 * j] = part[2 * j + 1] = 0.f;
+      if (start) return;  // the path's first pixel: nothing before it
+      float same[K], dn[K], up[K];  // flows to L_q(d), L_q(d-1), L_q(d+1)
+      float2 kept = make_float2(0.f, 0.f), side = kept, jumped = kept;
 #pragma unroll
-        for (int j = 1; j < K; ++j)
-          if (Lq[j] < mn) { mn = Lq[j]; mi = gl * K + j; }
-        const float mq = group_min<G>(mn);
-        const unsigned hit = (__ballot_sync(kFullMask, mn == mq) >> (grp * G)) & ((1u << G) - 1u);
-        const int kq = __shfl_sync(kFullMask, mi, grp * G + __ffs(hit) - 1);
-        // choices at p
-        float lm[K], lp[K];
-        neighbours<G, K>(Lq, gl, lm, lp);
-        const float jump = mq + P2;
-        float g1 = 0.f, g2 = 0.f, gall = 0.f;
-        float gsame[K], gm1[K], gp1v[K];
+      for (int t = 0; t < K; t += 2) {
+        float lo[2], hi[2], ju[2];
 #pragma unroll
-        for (int j = 0; j < K; ++j) {
-          float t = Lq[j];
-          int c3 = 0;
-          if (lm[j] + P1 < t) { t = lm[j] + P1; c3 = 1; }
-          if (lp[j] + P1 < t) { t = lp[j] + P1; c3 = 2; }
-          if (jump < t) { c3 = 3; }
-          gsame[j] = c3 == 0 ? gv[j] : 0.f;
-          gm1[j] = c3 == 1 ? gv[j] : 0.f;   // flows to L_q(d-1)
-          gp1v[j] = c3 == 2 ? gv[j] : 0.f;  // flows to L_q(d+1)
-          if (c3 == 1 || c3 == 2) g1 += gv[j];
-          if (c3 == 3) g2 += gv[j];
-          gall += gv[j];
+        for (int h = 0; h < 2; ++h) {
+          const int sh = code_shift<FK>(t + h, j);
+          const bool b0 = (w[(t + h) / 2] >> sh) & 1u, b1 = (w[(t + h) / 2] >> sh) & 2u;
+          const float v = gv[t + h];
+          lo[h] = b1 ? 0.f : v;  // codes 0 and 1
+          hi[h] = b1 ? v : 0.f;  // codes 2 and 3
+          same[t + h] = b0 ? 0.f : lo[h];
+          dn[t + h] = b0 ? lo[h] : 0.f;
+          up[t + h] = b0 ? 0.f : hi[h];
+          ju[h] = b0 ? hi[h] : 0.f;
         }
-        g1 = group_sum<G>(g1);
-        g2 = group_sum<G>(g2);
-        gall = group_sum<G>(gall);
-        if (ln.live && gl == 0) {
-          gp1[p] = g1;
-          gp2[p] = g2;
-        }
-        // gradient of L_q: same d, from d+1 choosing d-1 (i.e. d), from d-1 choosing d+1 (i.e. d)
-        const float from_up = __shfl_down_sync(kFullMask, gm1[0], 1);      // gm1 of d+1, for d = gl*8+7
-        const float from_down = __shfl_up_sync(kFullMask, gp1v[K - 1], 1); // gp1 of d-1, for d = gl*8
+        const float2 u = make_float2(up[t], up[t + 1]);
+        kept = __fadd2_rn(kept, __fadd2_rn(make_float2(lo[0], lo[1]), u));
+        side = __fadd2_rn(side, __fadd2_rn(make_float2(dn[t], dn[t + 1]), u));
+        jumped = __fadd2_rn(jumped, make_float2(ju[0], ju[1]));
+      }
+      part[2 * j] = side.x + side.y;
+      part[2 * j + 1] = jumped.x + jumped.y;
+      const float all_kept = group_sum<G>(kept.x + kept.y);
+      float from_up = __shfl_down_sync(kFullMask, dn[0], 1), from_dn = __shfl_up_sync(kFullMask, up[K - 1], 1);
+      if (gl == G - 1) from_up = 0.f;
+      if (gl == 0) from_dn = 0.f;
+      const int at = (int)((ar[j / 4] >> (8 * (j % 4))) & 0xffu) - gl * K;
 #pragma unroll
-        for (int j = 0; j < K; ++j) {
-          float v = gsame[j];
-          v += j < K - 1 ? gm1[j + 1] : (gl < G - 1 ? from_up : 0.f);
-          v += j > 0 ? gp1v[j - 1] : (gl > 0 ? from_down : 0.f);
-          if (gl * K + j == kq) v += g2 - gall;
-          gnext[j] = v;
-        }
+      for (int t = 0; t < K; ++t) {
+        float v = same[t] + (t < K - 1 ? dn[t + 1] : from_up);
+        v += t > 0 ? up[t - 1] : from_dn;
+        if (t == at) v -= all_kept;
+        gn[t] = v;
       }
     };
-    if (kr > 0 && nr == kSeg && na == kSeg) {
-      // both chains over a whole segment, away from the path's first pixel: fully unrolled, so
-      // the two steps of one iteration are one block of independent instructions
+    const int p0 = seg * kSeg;
+    const int start = down ? (seg == 0 ? kSeg - 1 : -1) : (seg == nseg - 1 ? len - 1 - p0 : -1);  // its slot
+    if (p0 + kSeg <= len && start < 0) {
 #pragma unroll
-      for (int i = 0; i < kSeg; ++i) {
-        r_step(i % kBwdPF, i, kSeg, std::false_type{});
-        a_step(i % kBwdPF, i, kSeg, std::false_type{});
-      }
+      for (int j = 0; j < kSeg; ++j) step_at(j, false);
     } else {
-      for (int i0 = 0; i0 < max(nr, na); i0 += kBwdPF) {
 #pragma unroll
-        for (int jr = 0; jr < kBwdPF; ++jr) {
-          const int i = i0 + jr;
-          if (i < nr) r_step(jr, i, nr, std::true_type{});
-          if (i < na) a_step(jr, i, na, std::true_type{});
-        }
+      for (int j = 0; j < kSeg; ++j) {
+        part[2 * j] = part[2 * j + 1] = 0.f;
+        if (position(seg, j) < len)
+          step_at(j, j == start);
+        else
+          fetch(j % PF, j + PF < kSeg ? si : si + 1, (j + PF) % kSeg);
       }
     }
-    __syncwarp();
+    reduce_segment<G>(part, gl);
+#pragma unroll
+    for (int i = 0; i < kSeg / G; ++i) {
+      const int pos = position(seg, gl * (kSeg / G) + i);
+      if (live && pos < len) {
+        gp1[base + pos * step] = part[2 * i];
+        gp2[base + pos * step] = part[2 * i + 1];
+      }
+    }
   }
 }
 
@@ -736,7 +761,8 @@ int cost_map(const float* cost, int B, int H, int W, int D, CUtensorMap* map) {
   return SGM_OK;
 }
 
-template <int K>
+// REC: the records (in ckpt) are written for a backward pass.
+template <int K, bool REC>
 int forward_impl(const float* cost, const float* p1, const float* p2, int B, int H, int W, float inv_t, float* sum,
                  float* ckpt, float* work, float* disp, cudaStream_t s) {
   constexpr int D = 32 * K;
@@ -748,20 +774,20 @@ int forward_impl(const float* cost, const float* p1, const float* p2, int B, int
   a.out[0] = sum;
   for (int i = 1; i < 4; ++i) a.out[i] = work + (i - 1) * V;
   const size_t slab = slab_elems(B, H, W, D);
-  for (int i = 0; i < 4; ++i) a.ckpt[i] = ckpt + slab * i;
+  for (int i = 0; i < 4; ++i) a.rec[i] = REC ? ckpt + slab * i : nullptr;
   a.q = make_grid<32>(B, H, W, D);
   CUtensorMap tm;
   int st = cost_map(cost, B, H, W, D, &tm);
   if (st) return st;
   constexpr size_t smem = fwd_smem_bytes<K>();
-  if (cudaFuncSetAttribute(k_float_fwd<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(k_float_fwd<K, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return check("float forward attribute");
-  k_float_fwd<K><<<a.q.first_block[4], kWarps * 32, smem, s>>>(tm, a);
+  k_float_fwd<K, REC><<<a.q.first_block[4], kWarps * 32, smem, s>>>(tm, a);
   st = check("float forward");
   if (st) return st;
   constexpr int GS = D / kK;  // lanes per pixel of the soft-argmin kernels
   const size_t px_per_block = 8 * (32 / GS);
-  k_soft_argmin_fwd<GS><<<(unsigned)((npix + px_per_block - 1) / px_per_block), 256, 0, s>>>(
+  k_soft_argmin_fwd<GS, REC><<<(unsigned)((npix + px_per_block - 1) / px_per_block), 256, 0, s>>>(
       sum, a.out[1], a.out[2], a.out[3], disp, npix, inv_t);
   return check("soft argmin");
 }
@@ -779,23 +805,17 @@ int backward_impl(const float* cost, const float* p1, const float* p2, int B, in
   int st = check("soft argmin backward");
   if (st) return st;
   BwdArgs a;
-  a.cost = cost;
-  a.p1 = p1;
-  a.p2 = p2;
   a.gsum = grad_sum;
   const size_t slab = slab_elems(B, H, W, D);
   float* maps = work + 3 * V;
   for (int i = 0; i < 4; ++i) {
-    a.ckpt[i] = ckpt + slab * i;
+    a.rec[i] = ckpt + slab * i;
     a.gout[i] = i == 0 ? grad_cost : work + (i - 1) * V;
     a.gp1[i] = maps + i * npix;
     a.gp2[i] = maps + (4 + i) * npix;
   }
   a.q = make_grid<G>(B, H, W, D);
-  constexpr size_t smem = bwd_smem_bytes<G, K>();
-  if (cudaFuncSetAttribute(k_float_bwd<G, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return check("float backward attribute");
-  k_float_bwd<G, K><<<a.q.first_block[4], kWarps * 32, smem, s>>>(a);
+  k_float_bwd<G, K><<<a.q.first_block[4], kWarps * 32, 0, s>>>(a);
   if ((st = check("float backward"))) return st;
   SumArgs r;
   r.g0 = reinterpret_cast<float4*>(grad_cost);
@@ -849,8 +869,19 @@ int sgm_float_forward(const float* cost, const float* p1, const float* p2, int32
     return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const float inv_t = 1.0f / temperature;
-  return D == 64 ? forward_impl<2>(cost, p1, p2, B, H, W, inv_t, sum, ckpt, work, disp, s)
-                 : forward_impl<1>(cost, p1, p2, B, H, W, inv_t, sum, ckpt, work, disp, s);
+  return D == 64 ? forward_impl<2, true>(cost, p1, p2, B, H, W, inv_t, sum, ckpt, work, disp, s)
+                 : forward_impl<1, true>(cost, p1, p2, B, H, W, inv_t, sum, ckpt, work, disp, s);
+}
+
+int sgm_float_disparity(const float* cost, const float* p1, const float* p2, int32_t B, int32_t H, int32_t W,
+                        int32_t D, float temperature, float* sum, float* work, float* disp, void* stream) {
+  int st = validate(B, H, W, D, temperature);
+  if (st || (st = check_present({cost, p1, p2, sum, work, disp})) || (st = check_aligned({cost, sum, work})))
+    return st;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const float inv_t = 1.0f / temperature;
+  return D == 64 ? forward_impl<2, false>(cost, p1, p2, B, H, W, inv_t, sum, nullptr, work, disp, s)
+                 : forward_impl<1, false>(cost, p1, p2, B, H, W, inv_t, sum, nullptr, work, disp, s);
 }
 
 int sgm_float_backward(const float* cost, const float* p1, const float* p2, int32_t B, int32_t H, int32_t W, int32_t D,

@@ -25,6 +25,8 @@ def _lib():
         lib.sgm_float_workspace_elems.restype = C.c_size_t
         lib.sgm_float_forward.argtypes = [vp, vp, vp, i32, i32, i32, i32, f32, vp, vp, vp, vp, vp]
         lib.sgm_float_forward.restype = i32
+        lib.sgm_float_disparity.argtypes = [vp, vp, vp, i32, i32, i32, i32, f32, vp, vp, vp, vp]
+        lib.sgm_float_disparity.restype = i32
         lib.sgm_float_backward.argtypes = [vp, vp, vp, i32, i32, i32, i32, f32, vp, vp, vp, vp, vp, vp, vp, vp, vp]
         lib.sgm_float_backward.restype = i32
         lib._float_sgm_bound = True
@@ -38,19 +40,25 @@ def _aligned(t):
 
 class FloatSGM(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, cost, p1, p2, temperature=1.0):
+    def forward(ctx, cost, p1, p2, temperature=1.0, grad_enabled=True):
         if not (cost.is_cuda and cost.dtype == torch.float32 and cost.dim() == 4):
             raise ValueError("cost must be a float32 CUDA tensor [B,H,W,D]")
         cost, p1, p2 = _aligned(cost.contiguous()), p1.contiguous().float(), p2.contiguous().float()
         B, H, W, D = cost.shape
         lib = _lib()
         sum_ = torch.empty_like(cost)
-        ckpt = torch.empty(lib.sgm_float_checkpoint_elems(B, H, W, D), dtype=torch.float32, device=cost.device)
         work = torch.empty(lib.sgm_float_workspace_elems(B, H, W, D), dtype=torch.float32, device=cost.device)
         disp = torch.empty((B, H, W), dtype=torch.float32, device=cost.device)
+        stream = torch.cuda.current_stream(cost.device).cuda_stream
+        if not (grad_enabled and any(ctx.needs_input_grad)):  # no backward pass: nothing to keep for it
+            st = lib.sgm_float_disparity(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D,
+                                         float(temperature), sum_.data_ptr(), work.data_ptr(), disp.data_ptr(), stream)
+            if st != 0:
+                raise RuntimeError(f"float SGM forward failed: {lib.sgm_last_error(None).decode()}")
+            return disp
+        ckpt = torch.empty(lib.sgm_float_checkpoint_elems(B, H, W, D), dtype=torch.float32, device=cost.device)
         st = lib.sgm_float_forward(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D, float(temperature),
-                                   sum_.data_ptr(), ckpt.data_ptr(), work.data_ptr(), disp.data_ptr(),
-                                   torch.cuda.current_stream(cost.device).cuda_stream)
+                                   sum_.data_ptr(), ckpt.data_ptr(), work.data_ptr(), disp.data_ptr(), stream)
         if st != 0:
             raise RuntimeError(f"float SGM forward failed: {lib.sgm_last_error(None).decode()}")
         ctx.save_for_backward(cost, p1, p2, sum_, ckpt)
@@ -74,11 +82,11 @@ class FloatSGM(torch.autograd.Function):
                                     torch.cuda.current_stream(cost.device).cuda_stream)
         if st != 0:
             raise RuntimeError(f"float SGM backward failed: {lib.sgm_last_error(None).decode()}")
-        return gcost, gp1, gp2, None
+        return gcost, gp1, gp2, None, None
 
 
 def float_sgm(cost, p1, p2, temperature: float = 1.0):
-    return FloatSGM.apply(cost, p1, p2, temperature)
+    return FloatSGM.apply(cost, p1, p2, temperature, torch.is_grad_enabled())
 
 
 def reference_sgm(cost, p1, p2, temperature: float = 1.0, return_sum: bool = False):

@@ -287,7 +287,7 @@ SGM_API int sgm_batch_bucket(sgm_batch_t b, int32_t index, sgm_batch_bucket_t* b
  * S = ((L_0 + L_1) + L_2) + L_3 over the paths (top->bottom, left->right, bottom->top,
  * right->left), disp = sum_d d*softmax(-S/T). Device pointers: cost [B][H][W][D],
  * p1/p2/disp [B][H][W], sum [B][H][W][D] (S, kept for the backward pass), ckpt of
- * sgm_float_checkpoint_elems floats (path states every 8 pixels, kept for the backward pass),
+ * sgm_float_checkpoint_elems floats (the choices of the path minima, kept for the backward pass),
  * work of sgm_float_workspace_elems floats (scratch, free after the call's work completes on
  * `stream`). D = 32 or 64; cost, sum, ckpt and work 16-byte aligned. */
 SGM_API size_t sgm_float_checkpoint_elems(int32_t B, int32_t H, int32_t W, int32_t D);
@@ -295,10 +295,14 @@ SGM_API size_t sgm_float_workspace_elems(int32_t B, int32_t H, int32_t W, int32_
 SGM_API int sgm_float_forward(const float* cost, const float* p1, const float* p2, int32_t B, int32_t H, int32_t W,
                               int32_t D, float temperature, float* sum, float* ckpt, float* work, float* disp,
                               void* stream);
+/* No counterpart in the reference. The disparity alone, for callers without a backward pass: the
+ * same disp as sgm_float_forward, without its records; sum and work are scratch. */
+SGM_API int sgm_float_disparity(const float* cost, const float* p1, const float* p2, int32_t B, int32_t H, int32_t W,
+                                int32_t D, float temperature, float* sum, float* work, float* disp, void* stream);
 /* No counterpart in the reference. Gradients of sum(grad_disp * disp) with respect to cost, p1
  * and p2 (written, not accumulated); grad_sum [B][H][W][D] and work (sgm_float_workspace_elems
- * floats) are scratch. Each path's states are recomputed from the checkpoints, 8 pixels at a
- * time. grad_sum and grad_cost 16-byte aligned. */
+ * floats) are scratch. Each path's gradient is routed by the recorded choices. grad_sum and
+ * grad_cost 16-byte aligned. */
 SGM_API int sgm_float_backward(const float* cost, const float* p1, const float* p2, int32_t B, int32_t H, int32_t W,
                                int32_t D, float temperature, const float* sum, const float* ckpt,
                                const float* grad_disp, float* grad_sum, float* work, float* grad_cost,

@@ -149,3 +149,68 @@ def test_fitting_penalty_maps_reduces_l1(oracle_mod):
         opt.step()
         losses.append(loss.item())
     assert losses[-1] < losses[0] * 0.98, losses[::10]
+
+
+def first_candidate_adjoint(cost, p1, p2, w):
+    """Disparity and gradients of sum(w * disp) in float64 with the documented order of equal
+    candidates (same d, d-1, d+1, jump; the lowest k of the minimum); autograd splits ties."""
+    D = cost.shape[-1]
+    pad = torch.nn.functional.pad
+
+    def candidates(q, m, a, b):
+        return torch.stack([q, pad(q, (1, 0), value=np.inf)[..., :-1] + a, pad(q, (0, 1), value=np.inf)[..., 1:] + a,
+                            (m + b).expand_as(q)])
+    disp, total = reference_sgm(cost, p1, p2, return_sum=True)
+    weight = torch.softmax(-total, -1)
+    g_sum = -w[..., None] * weight * (torch.arange(D, dtype=cost.dtype) - disp[..., None])
+    gc, g1, g2 = torch.zeros_like(cost), torch.zeros_like(p1), torch.zeros_like(p2)
+    for dim, rev in ((1, False), (2, False), (1, True), (2, True)):
+        order = list(range(cost.shape[dim]))[::-1 if rev else 1]
+        L = [cost.select(dim, order[0])]
+        for k in order[1:]:
+            m = L[-1].min(-1, keepdim=True).values
+            a, b = p1.select(dim, k)[..., None], p2.select(dim, k)[..., None]
+            L.append(cost.select(dim, k) + candidates(L[-1], m, a, b).min(0).values - m)
+        g = torch.zeros_like(L[0])
+        for i in range(len(order) - 1, -1, -1):
+            k = order[i]
+            g = g + g_sum.select(dim, k)
+            gc.select(dim, k).add_(g)
+            if i == 0:
+                break
+            q = L[i - 1]
+            m, at = q.min(-1, keepdim=True)
+            pick = candidates(q, m, p1.select(dim, k)[..., None], p2.select(dim, k)[..., None]).min(0).indices
+            same, dn, up, jump = (torch.where(pick == n, g, 0.0) for n in range(4))
+            g1.select(dim, k).add_((dn + up).sum(-1))
+            g2.select(dim, k).add_(jump.sum(-1))
+            back = same + pad(dn, (0, 1))[..., 1:] + pad(up, (1, 0))[..., :-1]
+            g = back.scatter_add(-1, at, jump.sum(-1, keepdim=True) - g.sum(-1, keepdim=True))
+    return disp, gc, g1, g2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("H,W", [(1, 1), (1, 9), (8, 1), (7, 8), (8, 16), (17, 33)])
+def test_segment_edges_and_disparity_alone(D, H, W):
+    """Lines that end before, at and past a segment (8) and a chunk (16): gradients against the FP64
+    adjoint, on half-integer costs and penalties so that equal candidates occur and every path sum is
+    exact; the call without gradients gives the same disparities."""
+    from fasterstereocuda_b200.float_sgm import float_sgm
+    gen = torch.Generator().manual_seed(100 * H + W + D)
+    c64 = torch.rand(2, H, W, D, generator=gen, dtype=torch.float64).argsort(-1).double() * 0.5
+    p1 = torch.randint(3, 7, (2, H, W), generator=gen).double() + 0.25
+    p2 = torch.randint(20, 40, (2, H, W), generator=gen).double() + 0.125
+    w = torch.randn(2, H, W, generator=gen, dtype=torch.float64)
+    c, q1, q2 = (t.float().cuda().requires_grad_() for t in (c64, p1, p2))
+    d = float_sgm(c, q1, q2)
+    (d * w.float().cuda()).sum().backward()
+    with torch.no_grad():
+        assert torch.equal(float_sgm(c, q1, q2), d)
+    dr, *expected = first_candidate_adjoint(c64, p1, p2, w)
+    assert torch.allclose(d.detach().cpu().double(), dr, rtol=1e-4, atol=1e-4)
+    for a, b, name in zip((c.grad, q1.grad, q2.grad), expected, ("cost", "p1", "p2")):
+        if b.norm() == 0:
+            assert a.abs().max() == 0, name
+            continue
+        assert (a.cpu().double() - b).norm() / b.norm() < 1e-3, name
