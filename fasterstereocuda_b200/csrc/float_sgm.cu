@@ -25,8 +25,7 @@
 // the adjoint routes the gradient of every L_p(d) to C_p(d), to P1(p) or P2(p) and to L_q by them.
 // Storing path states every 8 pixels and repeating the recurrence in the backward read the cost
 // volume a second time and ran the longer half of the backward's chain: 4 x 1242x375 x 64, scan
-// 1576 -> 772 us, with the recording forward scan at 640 us (645 before, 43.9 -> ~45 instructions a
-// step with the record, ~25 without it).
+// 1576 -> 772 us, with the recording forward scan at 640 us (645 before it).
 // Mapping, backward: a scanline is held by G lanes of a warp, 8 disparities per lane (8 lanes at
 // D = 64), sums by butterflies; the gradient of S is loaded kBwdPF steps ahead. Bound by DRAM:
 // 3.93 GB at 5.1 TB/s at that size.

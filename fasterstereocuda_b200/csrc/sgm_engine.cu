@@ -24,6 +24,7 @@
 #include "../../include/sgm_b200.h"
 #include "sgm_alloc.h"
 #include "sgm_kernels4.cuh"
+#include "sgm_kernels5.cuh"
 #include "sgm_levels.h"
 #include "sgm_tma.h"
 
@@ -209,8 +210,12 @@ struct sgm_engine {
   int tune_rows = 0;        // rows per CTA of the row kernels (0: default)
   int tune_cols = 0;        // columns per CTA of the column kernels (0: default)
   int tune_bt_smem = 0;     // 1: keep bottom->top path costs in shared memory when they fit
-  int tune_row_kernel = 0;  // 0: 3 when exact else 2; 1 whole-row census, 2 chunked, 3 u16x2 per scanline
-  int tune_col_kernel = 0;  // 0: 3 when exact else 1; 1 plain loads, 2 prefetch ring, 3 u16x2 per column
+  // 0: the default, else 1
+  // whole-row census, 2 chunked, 3 u16x2 per scanline, 4 one warp per scanline
+  int tune_row_kernel = 0;
+  // 0: the default, else 1 plain loads, 2 prefetch ring, 3 u16x2 per column, 4 one warp per column
+  int tune_col_kernel = 0;
+  bool latency = false;     // variant 4 in place of the default (see KernelMode)
   int tune_row_lanes = 0;   // variant 3: lanes per scanline (0: default)
   int tune_col_lanes = 0;
   bool bt_stored = true;    // the last match wrote the bottom->top volume to global memory
@@ -519,7 +524,8 @@ using sgm::EncodeTiledFn;
 using sgm::encode_tiled;
 
 // Tensor map i (0 cost, 1 bt, 2 lr, 3 rl, 4 tb) of the engine's volumes, [nv][H][W * D] bytes, in boxes
-// of 32 rows x D bytes with the D-byte swizzle (k_vscan_plain4); rebuilt when the volume moved.
+// of 32 rows x D bytes with the D-byte swizzle (k_vscan_plain4), at D = 256 of kC5 rows without
+// one (k_vscan_plain256); rebuilt when the volume moved.
 int volume_map(sgm_engine* e, int i, const uint8_t* base, int nv, const CUtensorMap** out) {
   sgm_engine::TmapKey& k = e->tmap_key[i];
   if (k.base != base || k.W != e->W || k.H != e->H || k.D != e->D || k.nv != nv) {
@@ -530,9 +536,10 @@ int volume_map(sgm_engine* e, int i, const uint8_t* base, int nv, const CUtensor
     }
     const cuuint64_t dims[3] = {(cuuint64_t)e->W * e->D, (cuuint64_t)e->H, (cuuint64_t)nv};
     const cuuint64_t strides[2] = {(cuuint64_t)e->W * e->D, (cuuint64_t)e->W * e->H * e->D};
-    const cuuint32_t box[3] = {(cuuint32_t)e->D, (cuuint32_t)sgm::kScanChunk, 1u};
+    const cuuint32_t box[3] = {(cuuint32_t)e->D, (cuuint32_t)(e->D == 256 ? sgm::kC5 : sgm::kScanChunk), 1u};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
-    const CUtensorMapSwizzle sw = e->D == 32   ? CU_TENSOR_MAP_SWIZZLE_32B
+    const CUtensorMapSwizzle sw = e->D == 256  ? CU_TENSOR_MAP_SWIZZLE_NONE
+                                  : e->D == 32   ? CU_TENSOR_MAP_SWIZZLE_32B
                                   : e->D == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
                                                : CU_TENSOR_MAP_SWIZZLE_128B;
     const CUresult r = fn(&e->tmap[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(base), dims, strides,
@@ -549,6 +556,11 @@ int volume_map(sgm_engine* e, int i, const uint8_t* base, int nv, const CUtensor
   return SGM_OK;
 }
 
+// Penalties for which the warp-per-scanline kernels run in 16-bit halves (plain_step16).
+bool narrow4_ok(const sgm::PlainParams& P) {
+  return P.p1 <= sgm::kInvalidCost && P.p1 <= P.p2 && P.p2 <= sgm::kMaxPenalty16;
+}
+
 // Warp-per-scanline kernels (variant 4, D <= 128): the row scans, and the column passes (pass 1
 // bottom-to-top, pass 2 top-to-bottom + sum + WTA).
 template <int K>
@@ -556,9 +568,14 @@ int launch_rows4(sgm_engine* e, const sgm::PlainParams& P, int nv, cudaStream_t 
   if constexpr (K <= 4) {
     constexpr int wpb = sgm::hscan_plain4_warps<K>();
     const int blocks = (nv * 2 * e->H + wpb - 1) / wpb;
-    SGM_CUDA_TRY(e, sgm::prefer_max_shared(sgm::k_hscan_plain4<K>));
-    return SGM_LAUNCH(e, s, "hpaths_plain",
-                      sgm::k_hscan_plain4<K><<<blocks, 32 * wpb, 0, s>>>(e->cost, e->lr, e->rl, P, nv));
+    auto go = [&](auto kern) -> int {
+      SGM_CUDA_TRY(e, sgm::prefer_max_shared(kern));
+      return SGM_LAUNCH(e, s, "hpaths_plain", kern<<<blocks, 32 * wpb, 0, s>>>(e->cost, e->lr, e->rl, P, nv));
+    };
+    if constexpr (K >= 2) {
+      if (narrow4_ok(P)) return go(sgm::k_hscan_plain4<K, true>);
+    }
+    return go(sgm::k_hscan_plain4<K, false>);
   } else {
     return SGM_ERR_UNSUPPORTED;
   }
@@ -577,6 +594,30 @@ int ensure_tb(sgm_engine* e, int nv) {
   return SGM_OK;
 }
 
+// D = 256 (sgm_kernels5.cuh).
+inline int launch_rows256(sgm_engine* e, const sgm::PlainParams& P, int nv, cudaStream_t s) {
+  constexpr int wpb = sgm::kWpb5;
+  SGM_CUDA_TRY(e, sgm::prefer_max_shared(sgm::k_hscan_plain256));
+  return SGM_LAUNCH(e, s, "hpaths_plain", sgm::k_hscan_plain256<<<(nv * 2 * e->H + wpb - 1) / wpb, 32 * wpb, 0, s>>>(
+                                              e->cost, e->lr, e->rl, P, nv));
+}
+
+template <int PASS>
+int launch_cols256(sgm_engine* e, const sgm::PlainParams& P, const sgm::WtaParams& Q, float* wta, int nv,
+                   cudaStream_t s) {
+  const dim3 grid((e->W + sgm::kWpb5 - 1) / sgm::kWpb5, nv);
+  const CUtensorMap *mc, *mb, *ml, *mr;
+  int st = volume_map(e, 0, e->cost, nv, &mc);
+  if (!st) st = volume_map(e, 1, e->bt, nv, &mb);
+  if (!st) st = volume_map(e, 2, e->lr, nv, &ml);
+  if (!st) st = volume_map(e, 3, e->rl, nv, &mr);
+  if (st) return st;
+  SGM_CUDA_TRY(e, sgm::prefer_max_shared(sgm::k_vscan_plain256<PASS>));
+  return SGM_LAUNCH(e, s, PASS == 1 ? "vpaths_bt_plain" : "vpaths_wta_plain",
+                    sgm::k_vscan_plain256<PASS><<<grid, 32 * sgm::kWpb5, sgm::vscan256_smem<PASS>(), s>>>(
+                        *mc, *mb, *ml, *mr, e->bt, wta, P, Q));
+}
+
 template <int K, int PASS>
 int launch_cols4(sgm_engine* e, const sgm::PlainParams& P, const sgm::WtaParams& Q, float* wta, int nv,
                  cudaStream_t s) {
@@ -589,9 +630,15 @@ int launch_cols4(sgm_engine* e, const sgm::PlainParams& P, const sgm::WtaParams&
     if (!st) st = volume_map(e, 2, e->lr, nv, &ml);
     if (!st) st = volume_map(e, 3, e->rl, nv, &mr);
     if (st) return st;
-    SGM_CUDA_TRY(e, sgm::prefer_max_shared(sgm::k_vscan_plain4<K, PASS>));
-    return SGM_LAUNCH(e, s, PASS == 1 ? "vpaths_bt_plain" : "vpaths_wta_plain",
-                      sgm::k_vscan_plain4<K, PASS><<<grid, 32 * wpb, 0, s>>>(*mc, *mb, *ml, *mr, e->bt, wta, P, Q));
+    auto go = [&](auto kern) -> int {
+      SGM_CUDA_TRY(e, sgm::prefer_max_shared(kern));
+      return SGM_LAUNCH(e, s, PASS == 1 ? "vpaths_bt_plain" : "vpaths_wta_plain",
+                        kern<<<grid, 32 * wpb, 0, s>>>(*mc, *mb, *ml, *mr, e->bt, wta, P, Q));
+    };
+    if constexpr (K >= 2) {
+      if (narrow4_ok(P)) return go(sgm::k_vscan_plain4<K, PASS, true>);
+    }
+    return go(sgm::k_vscan_plain4<K, PASS, false>);
   } else {
     return SGM_ERR_UNSUPPORTED;
   }
@@ -629,17 +676,21 @@ int launch_plain(sgm_engine* e, const Word* csl, const Word* csr, float* wta) {
   P.p1 = (uint32_t)e->opt.p1; P.p2 = (uint32_t)e->opt.p2_init;
   P.vstride = e->vol();
   const int nv = e->nviews();
-  // thread-per-scanline kernels: exact for 16-bit path costs and the min(x + P1, L) form
-  const bool v3_ok = K <= 4 && e->opt.p1 <= (int)sgm::kMaxPenalty16 && e->opt.p2_init <= (int)sgm::kMaxPenalty16 &&
-                     e->opt.p2_init >= e->opt.p1 &&
-                     (e->ext.tie_rule == sgm::kTieLowest || e->ext.tie_rule == sgm::kTieRefB200);
+  // 16-bit path costs and the min(x + P1, L) form are exact
+  const bool narrow_ok = e->opt.p1 <= (int)sgm::kMaxPenalty16 && e->opt.p2_init <= (int)sgm::kMaxPenalty16 &&
+                         e->opt.p2_init >= e->opt.p1 &&
+                         (e->ext.tie_rule == sgm::kTieLowest || e->ext.tie_rule == sgm::kTieRefB200);
+  const bool v3_ok = K <= 4 && narrow_ok;
   int st;
   // warp-per-scanline kernels: D <= 128 and the tie rules of their serial WTA; otherwise the
   // default takes their place
   const bool v4_ok = K <= 4 && (e->ext.tie_rule == sgm::kTieLowest || e->ext.tie_rule == sgm::kTieHighest ||
                                 e->ext.tie_rule == sgm::kTieRefB200);
-  const int tune_row = e->tune_row_kernel == 4 && !v4_ok ? 0 : e->tune_row_kernel;
-  const int tune_col = e->tune_col_kernel == 4 && !v4_ok ? 0 : e->tune_col_kernel;
+  const bool by_default = e->tuning_is_default();
+  const int want_row = by_default && e->latency ? 4 : e->tune_row_kernel;
+  const int want_col = by_default && e->latency ? 4 : e->tune_col_kernel;
+  const int tune_row = want_row == 4 && !v4_ok ? 0 : want_row;
+  const int tune_col = want_col == 4 && !v4_ok ? 0 : want_col;
   const bool cols_v3 = (tune_col == 3 || tune_col == 0) && v3_ok;
   const bool cols_v4 = tune_col == 4;
   sgm::WtaParams Q;
@@ -650,6 +701,16 @@ int launch_plain(sgm_engine* e, const Word* csl, const Word* csr, float* wta) {
   Q.dmax_excl = warp_kernel ? 32 * K : 32 * K - 1;
   Q.dstride = e->npix();
   Q.image_border(e->W, e->H);
+  if (K == 8 && by_default && narrow_ok && narrow4_ok(P)) {
+    dim3 cg((e->W + 127) / 128, e->H, nv);
+    st = SGM_LAUNCH(e, e->stream, "cost", sgm::k_cost3<K, Word><<<cg, 128, 0, e->stream>>>(csl, csr, e->cost, P));
+    e->bt_stored = true;
+    if (!st)
+      st = fork_join(
+          e, e->stream, [&](cudaStream_t ss) { return launch_cols256<1>(e, P, Q, wta, nv, ss); },
+          [&](cudaStream_t ms) { return launch_rows256(e, P, nv, ms); });
+    return st ? st : launch_cols256<2>(e, P, Q, wta, nv, e->stream);
+  }
   if (((tune_row == 3 || tune_row == 0) && v3_ok) || tune_row == 4) {
     dim3 cg((e->W + 127) / 128, e->H, nv);
     st = SGM_LAUNCH(e, e->stream, "cost", sgm::k_cost3<K, Word><<<cg, 128, 0, e->stream>>>(csl, csr, e->cost, P));
@@ -945,10 +1006,12 @@ int launch_init(sgm_engine* e, const Word* csl, const Word* csr, const int16_t* 
   const bool v3_ok = e->ext.init_tie_rule == sgm::kTieLowest || e->ext.init_tie_rule == sgm::kTieRefB200;
   // the warp-per-scanline row kernel packs P2' into 22 bits; larger penalties take the default
   const bool pack_ok = e->opt.p1 >= 0 && e->opt.p1 < (1 << 22) && e->opt.p2_init < (1 << 22) && e->ext.p2_div0 < (1 << 22);
-  const int tune_row = e->tune_row_kernel == 4 && !pack_ok ? 0 : e->tune_row_kernel;
+  const bool lat = e->latency && e->tuning_is_default();
+  const int want_row = lat ? 4 : e->tune_row_kernel, tune_col = lat ? 4 : e->tune_col_kernel;
+  const int tune_row = want_row == 4 && !pack_ok ? 0 : want_row;
   const bool rows3 = v3_ok && (tune_row == 0 || tune_row == 3);
-  const bool cols3 = v3_ok && (e->tune_col_kernel == 0 || e->tune_col_kernel == 3);
-  const bool rows4 = tune_row == 4, cols4 = e->tune_col_kernel == 4;
+  const bool cols3 = v3_ok && (tune_col == 0 || tune_col == 3);
+  const bool rows4 = tune_row == 4, cols4 = tune_col == 4;
   // rows reading the cost volume (variants 3 and 4) and columns split into two passes
   auto rows_cv = [&](cudaStream_t ms) { return rows4 ? init4_rows(e, il, ir, P, ms) : init3_rows(e, il, ir, P, ms); };
   auto cols_bt = [&](cudaStream_t ss) {
@@ -1006,7 +1069,7 @@ int launch_init(sgm_engine* e, const Word* csl, const Word* csr, const int16_t* 
     st = init4_cols_both(e, il, ir, P, e->stream);
     return st ? st : init4_wta(e, il, ir, wta, P, Q3, e->stream);
   }
-  if (e->tune_col_kernel != 2) {
+  if (tune_col != 2) {
     C = e->tune_cols > 0 ? e->tune_cols : 8;
     e->bt_stored = true;
     dim3 vg((e->W + C - 1) / C, nv), vb(32, C);
@@ -1300,8 +1363,8 @@ struct HostCall {
   bool (*poll() const)() { return latency() ? few_host_calls : nullptr; }
 };
 
-// Row and column kernels set to variant 4 on the given engines for the scope of one match, when
-// `latency` and every engine is at the default tuning; mode() is the graph slot to use.
+// Latency kernels on the given engines for the scope of one match, when `latency` and every engine
+// is at the default tuning; mode() is the graph slot to use.
 struct KernelMode {
   sgm_engine* const* lv;
   int n;
@@ -1311,11 +1374,11 @@ struct KernelMode {
     for (int i = 0; i < n; ++i)
       if (!lv[i]->tuning_is_default()) return;
     on = true;
-    for (int i = 0; i < n; ++i) lv[i]->tune_row_kernel = lv[i]->tune_col_kernel = 4;
+    for (int i = 0; i < n; ++i) lv[i]->latency = true;
   }
   ~KernelMode() {
     if (on)
-      for (int i = 0; i < n; ++i) lv[i]->tune_row_kernel = lv[i]->tune_col_kernel = 0;
+      for (int i = 0; i < n; ++i) lv[i]->latency = false;
   }
   KernelMode(const KernelMode&) = delete;
   KernelMode& operator=(const KernelMode&) = delete;

@@ -494,27 +494,119 @@ __device__ __forceinline__ void plain_step4(uint32_t (&L)[K], const uint32_t (&c
   }
 }
 
+// The same recurrence in 16-bit halves: lane l holds its K disparities as K / 2 words (u16x2), exact
+// for P1 <= 127, P1 <= P2 <= 16383 (host: narrow4_ok). A GPU full of scans is bound by the integer ALU
+// (DPX minima, byte permutes and selects all issue at half rate), so what counts is ALU operations
+// per step: about 10 instead of 15 at K = 2, 19 instead of 29 at K = 4. 1242x375, D = 64, one pair
+// alone: rows 110 -> 92 us, columns 47 + 66 -> 39 + 60 us; 32 pairs in flight 166 -> 153 us a pair
+// (D = 128, 957x541: 344 -> 294 us). Two things keep the count down:
+//   * the minimum over the lane's halves is taken in both halves (min(v, v with halves swapped)),
+//     so one REDUX returns m in both halves and m never has to be spread;
+//   * the candidate 127 beyond d = 0 and d = D - 1 rides on the jump candidate: x is
+//     min(L(d-1), L(d+1), min(m + P2 - P1, cap)) with cap = 127 - P1 there, and x + P1 follows. At
+//     K = 2 the edge lanes' shuffles return the lane's own word, whose half is the other neighbour, a
+//     candidate anyway; wider lanes put all ones there (sgm_kernels5.cuh holds eight disparities a lane the same way).
+struct Consts16 {
+  uint32_t p1x2, p2m1x2, cap_lo, cap_hi;  // cap of the lane's first and last word (K = 2: both in cap_lo)
+};
+template <int K>
+__device__ __forceinline__ Consts16 consts16(uint32_t p1, uint32_t p2) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t cap = (kInvalidCost - p1) & 0xFFFFu;
+  Consts16 q;
+  q.p1x2 = rep16(p1);
+  q.p2m1x2 = rep16(p2 - p1);
+  q.cap_lo = lane == 0 ? 0xFFFF0000u | cap : 0xFFFFFFFFu;
+  q.cap_hi = lane == 31 ? (cap << 16) | 0xFFFFu : 0xFFFFFFFFu;
+  if (K == 2) q.cap_lo &= q.cap_hi;
+  return q;
+}
+// min over the scanline of L, in both halves
+template <int NW>
+__device__ __forceinline__ uint32_t min16_both(const uint32_t (&L)[NW]) {
+  uint32_t v = L[0];
+  if constexpr (NW == 2) v = min16x2(L[0], L[1]);
+  if constexpr (NW == 4) v = min16x2(__vimin3_u16x2(L[0], L[1], L[2]), L[3]);
+  return __reduce_min_sync(kFull, min16x2(v, __byte_perm(v, v, 0x1032)));
+}
+// mm: m in both halves, of the state before and after the step
+template <int NW>
+__device__ __forceinline__ void plain_step16(uint32_t (&L)[NW], const uint32_t (&c)[NW], uint32_t& mm,
+                                             const Consts16& q) {
+  const int lane = threadIdx.x & 31;
+  uint32_t ln = __shfl_up_sync(kFull, L[NW - 1], 1), rn = __shfl_down_sync(kFull, L[0], 1);
+  if constexpr (NW > 1) {
+    ln = lane == 0 ? 0xFFFFFFFFu : ln;
+    rn = lane == 31 ? 0xFFFFFFFFu : rn;
+  }
+  uint32_t b[NW + 1];  // b[k], b[k + 1]: the words of d - 1 and d + 1 of word k
+  b[0] = __byte_perm(ln, L[0], 0x5432);
+#pragma unroll
+  for (int k = 1; k < NW; ++k) b[k] = __byte_perm(L[k - 1], L[k], 0x5432);
+  b[NW] = __byte_perm(L[NW - 1], rn, 0x5432);
+  // m + P2 - P1 (no half reaches 2^16), capped where the word holds an end of the range
+  const uint32_t first = __viaddmin_u16x2(mm, q.p2m1x2, q.cap_lo);
+  const uint32_t last = NW > 1 ? __viaddmin_u16x2(mm, q.p2m1x2, q.cap_hi) : first;
+  const uint32_t mid = NW > 2 ? mm + q.p2m1x2 : 0u;
+#pragma unroll
+  for (int k = 0; k < NW; ++k) {
+    const uint32_t x = __vimin3_u16x2(b[k], b[k + 1], k == 0 ? first : (k == NW - 1 ? last : mid));
+    L[k] = __viaddmin_u16x2(x, q.p1x2, L[k]) + c[k] - mm;
+  }
+  mm = min16_both<NW>(L);
+}
+
+// The state of a scanline: 32-bit costs, or 16-bit halves and their minimum.
+template <int K, bool N16>
+struct Plain4 {
+  uint32_t L[N16 ? K / 2 : K], mm = 0;
+  Consts16 q;
+  uint32_t p1, p2;
+  __device__ __forceinline__ Plain4(const PlainParams& P) : p1(P.p1), p2(P.p2) {
+    if constexpr (N16) q = consts16<K>(P.p1, P.p2);
+  }
+  // one step from the lane's K cost bytes; start: L = C
+  __device__ __forceinline__ uint32_t advance(uint32_t w, bool start) {
+    if constexpr (N16) {
+      uint32_t c[K / 2];
+      c[0] = widen_lo(w);
+      if constexpr (K == 4) c[1] = widen_hi(w);
+      if (start) {
+#pragma unroll
+        for (int k = 0; k < K / 2; ++k) L[k] = c[k];
+        mm = min16_both<K / 2>(L);
+      } else {
+        plain_step16<K / 2>(L, c, mm, q);
+      }
+      return K == 4 ? narrow(L[0], L[K / 2 - 1]) : __byte_perm(L[0], 0u, 0x4420);
+    } else {
+      uint32_t c[K];
+      unpack_bytes<K>(w, c);
+      if (start) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) L[k] = c[k];
+      } else {
+        plain_step4<K>(L, c, p1, p2);
+      }
+      return pack_bytes<K>(L);
+    }
+  }
+};
+
 // The 32 steps of a chunk held in shared memory: at step j this lane reads its K bytes of costs
 // at at(j) (a LaneBytes<K> pointer) and leaves its path costs there. first: step 0 starts the
 // scanline (L = C). Costs are read R steps ahead.
-template <int K, typename At>
-__device__ __forceinline__ void plain_chunk(At at, bool first, uint32_t (&L)[K], uint32_t p1, uint32_t p2) {
+template <int K, bool N16, typename At>
+__device__ __forceinline__ void plain_chunk(At at, bool first, Plain4<K, N16>& st) {
   constexpr int C = kScanChunk, R = 16;
   uint32_t ring[R];
 #pragma unroll
   for (int j = 0; j < R; ++j) ring[j] = *at(j);
 #pragma unroll
   for (int j = 0; j < C; ++j) {
-    uint32_t c[K];
-    unpack_bytes<K>(ring[j % R], c);
+    const uint32_t w = ring[j % R];
     if (j + R < C) ring[j % R] = *at(j + R);
-    if (j == 0 && first) {
-#pragma unroll
-      for (int k = 0; k < K; ++k) L[k] = c[k];
-    } else {
-      plain_step4<K>(L, c, p1, p2);
-    }
-    *at(j) = (LaneBytes<K>)pack_bytes<K>(L);
+    *at(j) = (LaneBytes<K>)st.advance(w, j == 0 && first);
   }
 }
 
@@ -525,7 +617,7 @@ __device__ __forceinline__ void plain_chunk(At at, bool first, uint32_t (&L)[K],
 template <int K>
 __host__ __device__ constexpr int hscan_plain4_warps() { return K == 4 ? 2 : 4; }
 
-template <int K, int WPB = hscan_plain4_warps<K>()>
+template <int K, bool N16, int WPB = hscan_plain4_warps<K>()>
 __global__ void __launch_bounds__(32 * WPB) k_hscan_plain4(const uint8_t* __restrict__ cost, uint8_t* __restrict__ lr,
                                                            uint8_t* __restrict__ rl, PlainParams P, int nviews) {
   constexpr int D = 32 * K, C = kScanChunk, NB = 3;
@@ -562,7 +654,7 @@ __global__ void __launch_bounds__(32 * WPB) k_hscan_plain4(const uint8_t* __rest
     if (nch > 1) issue(1);
   }
   uint32_t phase = 0u;
-  uint32_t L[K];
+  Plain4<K, N16> st(P);
   for (int c = 0; c < nch; ++c) {
     const int b = c % NB, n = chunk_n(c);
     if (!mbar_wait_warp(&bars[w][b], (phase >> b) & 1u)) {
@@ -574,9 +666,9 @@ __global__ void __launch_bounds__(32 * WPB) k_hscan_plain4(const uint8_t* __rest
     __syncwarp();
     LaneBytes<K>* lb = reinterpret_cast<LaneBytes<K>*>(cbuf[w][b]) + lane;
     if (dir == 0)
-      plain_chunk<K>([lb](int j) { return lb + j * 32; }, c == 0, L, P.p1, P.p2);
+      plain_chunk<K, N16>([lb](int j) { return lb + j * 32; }, c == 0, st);
     else
-      plain_chunk<K>([lb](int j) { return lb + (C - 1 - j) * 32; }, c == 0, L, P.p1, P.p2);
+      plain_chunk<K, N16>([lb](int j) { return lb + (C - 1 - j) * 32; }, c == 0, st);
     fence_proxy_async();  // the chunk's path costs (and its cost reads) before the bulk copies
     __syncwarp();
     if (lane == 0) {
@@ -685,7 +777,7 @@ __host__ __device__ constexpr int vscan_plain4_warps() { return K == 4 ? 2 : 4; 
 // top to bottom over boxes starting at rows 32c, then per box the WTA of its pixels with lane =
 // pixel (rows >= Q.rows INVALID, as the reference's two-row WTA blocks leave them; border and
 // columns left of x0 INVALID). Maps: the cost, bt, lr and rl volumes, [views][H][W * D] bytes.
-template <int K, int PASS>
+template <int K, int PASS, bool N16>
 __global__ void __launch_bounds__(32 * vscan_plain4_warps<K>())
     k_vscan_plain4(const __grid_constant__ CUtensorMap m_cost, const __grid_constant__ CUtensorMap m_bt,
                    const __grid_constant__ CUtensorMap m_lr, const __grid_constant__ CUtensorMap m_rl,
@@ -740,7 +832,7 @@ __global__ void __launch_bounds__(32 * vscan_plain4_warps<K>())
 #pragma unroll
   for (int v = 0; v < NSW; ++v) lane_off[v] = (K * lane) ^ (v << 4);
   uint32_t phase = 0u;  // bit b: parity awaited on bars[w][b]
-  uint32_t L[K];
+  Plain4<K, N16> st(P);
   const bool col_ok = x >= Q.xlo && x <= Q.xhi;
   for (int c = 0; c < nch; ++c) {
     const int b = c % NB;
@@ -754,12 +846,12 @@ __global__ void __launch_bounds__(32 * vscan_plain4_warps<K>())
     __syncwarp();
     uint8_t* box = cbuf[w][b];
     // step j: box row C - 1 - j (PASS 1) or j (PASS 2)
-    plain_chunk<K>(
+    plain_chunk<K, N16>(
         [&](int j) {
           const int r = PASS == 1 ? C - 1 - j : j;
           return reinterpret_cast<LaneBytes<K>*>(box + r * D + lane_off[box_sw<D>(r)]);
         },
-        c == 0, L, P.p1, P.p2);
+        c == 0, st);
     if constexpr (PASS == 1) {
       fence_proxy_async();
       __syncwarp();
