@@ -378,6 +378,7 @@ __global__ void __launch_bounds__(128, G == 2 ? 5 : 1)
   constexpr int S = 32 / G;
   __shared__ uint32_t p2tab[sgm::kP2Tab];
   __shared__ uint32_t rows[sgm::init_rs<G>() * sgm::kIRow];
+  __shared__ __align__(16) uint8_t ring[4][sgm::CopyRing<sgm::kLevelRange / G / 4, PF>::kWarpBytes];
   init_scan_smem<G>(p2tab, rows, pairs[__ldg(ids)].IP);
   uint32_t* row = rows + threadIdx.x / G;
   const int lane = threadIdx.x & 31;
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(128, G == 2 ? 5 : 1)
     const BatchPair d = pairs[__ldg(ids + b)];
     const int local = item - __ldg(prefix + b);
     sgm::hpaths3_init_lane<G, PF>(d.cost, d.init, d.init, d.lr, d.rl, d.IP, d.nv, local * S + lane / G, lane % G, row,
-                                  p2tab);
+                                  p2tab, ring[threadIdx.x >> 5]);
   }
 }
 

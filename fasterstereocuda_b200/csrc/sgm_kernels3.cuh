@@ -64,6 +64,54 @@ __device__ __forceinline__ void st_slice(uint8_t* __restrict__ p, const uint32_t
   }
 }
 
+// A lane's slices of the next PF steps, in shared memory: its own asynchronous copies (cp.async, one
+// group per step), read back by itself, so no barrier is needed. A ring of PF registers loads as far
+// ahead on paper, but a warp's loads and shuffles share a few scoreboards: a step that waits for the
+// oldest load waits for younger ones on the same scoreboard, up to the one just issued. The copy
+// groups retire in order, and the step waits for its own alone. For the row scans of the
+// 32-disparity levels, whose two lanes a scanline copy one 32-byte sector a step: 64 pyramids of
+// 1242x375, both levels 2292 -> 1618 us. Not for the plain levels (eight pairs of 1242x375, D = 64:
+// 1485 -> 1870 us a batch: their lanes' 32 bytes a step are two half-sector copies each).
+template <int NR, int PF>
+struct CopyRing {
+  static constexpr int kUnit = NR >= 4 ? 16 : 4 * NR, kUnits = NR >= 4 ? NR / 4 : 1;
+  static constexpr int kWarpBytes = PF * 128 * NR;
+  uint8_t* mine;  // this lane's first unit of slot 0; a warp's accesses of a unit are contiguous
+  __device__ __forceinline__ explicit CopyRing(void* warp_base)
+      : mine(static_cast<uint8_t*>(warp_base) + (threadIdx.x & 31) * kUnit) {}
+  // The slice at src into `slot`, or nothing; a group either way.
+  __device__ __forceinline__ void copy(int slot, const uint8_t* src, bool pred) const {
+    if (pred) {
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(mine + slot * 128 * NR);
+#pragma unroll
+      for (int u = 0; u < kUnits; ++u) {
+        if constexpr (kUnit == 16)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + u * 512), "l"(src + u * 16) : "memory");
+        else
+          asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(kUnit) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // Waits until all but the newest PF - 1 groups are there and reads `slot`.
+  __device__ __forceinline__ void take(int slot, uint32_t (&r)[NR]) const {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PF - 1) : "memory");
+    const uint8_t* p = mine + slot * 128 * NR;
+    if constexpr (NR == 1) {
+      r[0] = *reinterpret_cast<const uint32_t*>(p);
+    } else if constexpr (NR == 2) {
+      const uint2 q = *reinterpret_cast<const uint2*>(p);
+      r[0] = q.x; r[1] = q.y;
+    } else {
+#pragma unroll
+      for (int u = 0; u < kUnits; ++u) {
+        const uint4 q = *reinterpret_cast<const uint4*>(p + u * 512);
+        r[4 * u] = q.x; r[4 * u + 1] = q.y; r[4 * u + 2] = q.z; r[4 * u + 3] = q.w;
+      }
+    }
+  }
+};
+
 // Bulk prefetch of `bytes` (a multiple of 16, 16-byte aligned, inside one allocation) into L2.
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
@@ -71,13 +119,14 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
 
 // A row scan reads one short slice per row and step, so its loads of one DRAM page are spread
 // over many steps. Every 16 steps the scanline's first lane prefetches the row's next 16 pixels
-// (steps s0 + 8 .. s0 + 23, clamped to the scanline) into L2 in one request.
+// (steps s0 + ahead .. s0 + ahead + 15, clamped to the scanline) into L2 in one request.
 // With many pairs in flight: +3.5 % pyramid, +7.5 % plain pairs/s (a single pair's scans alone
 // run ~10 % faster without it).
 template <int BYTES_PER_PX>
-__device__ __forceinline__ void prefetch_row_ahead(const uint8_t* row, int xs, int dx, int s0, int len, int g) {
+__device__ __forceinline__ void prefetch_row_ahead(const uint8_t* row, int xs, int dx, int s0, int len, int g,
+                                                   int ahead = 8) {
   if (g == 0 && (s0 & 15) == 0) {
-    const int a = s0 + 8, n = min(16, len - a);
+    const int a = s0 + ahead, n = min(16, len - a);
     if (n > 0) {
       const int x_lo = dx > 0 ? xs + a : xs - a - (n - 1);
       prefetch_l2(row + (size_t)x_lo * BYTES_PER_PX, (uint32_t)(n * BYTES_PER_PX));
@@ -1000,7 +1049,7 @@ __device__ __forceinline__ void hpaths3_init_lane(const uint8_t* __restrict__ co
                                                   const int16_t* __restrict__ init_l,
                                                   const int16_t* __restrict__ init_r, uint8_t* __restrict__ lr,
                                                   uint8_t* __restrict__ rl, const InitParams& P, int nviews, int i,
-                                                  int g, uint32_t* row, const uint32_t* p2tab) {
+                                                  int g, uint32_t* row, const uint32_t* p2tab, void* warp_ring) {
   constexpr int ND = kLevelRange / G, NR = ND / 4;
   const int H = P.H, W = P.W;
   const int nscan = nviews * 2 * H;
@@ -1020,35 +1069,35 @@ __device__ __forceinline__ void hpaths3_init_lane(const uint8_t* __restrict__ co
   uint32_t L[ND], out[NR];
   uint32_t m = 0;
   int last_base = 0;
-  // 16-bit steps with a PF-deep prefetch ring up to s_wide, 32-bit steps (plain loads) after it
+  // 16-bit steps with costs copied PF steps ahead up to s_wide, 32-bit steps (plain loads) after it
   int s_wide = init_narrow_ok(P) ? len : 0;
   static_assert(PF <= kNarrowBlock, "the 16-bit bound holds for kNarrowBlock steps");
   static_assert(16 % PF == 0, "blocks of PF steps start every 16 steps");
   if (s_wide > 0) {
-    uint32_t ring[PF][NR];
-    int rbase[PF];
+    const CopyRing<NR, PF> ring(warp_ring);
+    int next[PF];  // bases of the next block, loaded a block ahead
 #pragma unroll
     for (int j = 0; j < PF; ++j) {
-      if (j < len) {
-        ld_slice<NR>(crow + (size_t)(xs + j * dx) * kLevelRange, ring[j]);
-        rbase[j] = ib[xs + j * dx];
-      }
+      ring.copy(j, crow + (ptrdiff_t)(xs + j * dx) * kLevelRange, j < len);
+      next[j] = j < len ? ib[xs + j * dx] : 0;
     }
     for (int s0 = 0; s0 < s_wide; s0 += PF) {
-      prefetch_row_ahead<kLevelRange>(crow - (size_t)g * ND, xs, dx, s0, len, g);
+      int rbase[PF];
+#pragma unroll
+      for (int j = 0; j < PF; ++j) {
+        rbase[j] = next[j];
+        if (s0 + PF + j < len) next[j] = ib[xs + (s0 + PF + j) * dx];
+      }
+      prefetch_row_ahead<kLevelRange>(crow - (size_t)g * ND, xs, dx, s0, len, g, PF + 8);
 #pragma unroll
       for (int j = 0; j < PF; ++j) {
         const int s = s0 + j;
         if (s < s_wide) {
           const int x = xs + s * dx;
           uint32_t r[NR];
-#pragma unroll
-          for (int k = 0; k < NR; ++k) r[k] = ring[j][k];
+          ring.take(j, r);
           const int base = rbase[j];
-          if (s + PF < len) {
-            ld_slice<NR>(crow + (size_t)(x + PF * dx) * kLevelRange, ring[j]);
-            rbase[j] = ib[x + PF * dx];
-          }
+          ring.copy(j, crow + (ptrdiff_t)(x + PF * dx) * kLevelRange, s + PF < len);
           if (s == 0) {
             m = init_first<ND, G>(L, r, false);
             last_base = base;
@@ -1091,12 +1140,14 @@ __global__ void __launch_bounds__(128) k_hpaths3_init(const uint8_t* __restrict_
                                                       uint8_t* __restrict__ rl, InitParams P, int nviews) {
   __shared__ uint32_t p2tab[kP2Tab];
   __shared__ uint32_t rows[init_rs<G>() * kIRow];
+  __shared__ __align__(16) uint8_t ring[4][CopyRing<kLevelRange / G / 4, PF>::kWarpBytes];
   fill_p2_table(p2tab, P, threadIdx.x, blockDim.x);
   uint32_t* row = rows + threadIdx.x / G;
   init_row_pad<G>(row, P.p1, true, threadIdx.x % G);
   __syncthreads();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  hpaths3_init_lane<G, PF>(cost, init_l, init_r, lr, rl, P, nviews, t / G, threadIdx.x % G, row, p2tab);
+  hpaths3_init_lane<G, PF>(cost, init_l, init_r, lr, rl, P, nviews, t / G, threadIdx.x % G, row, p2tab,
+                           ring[threadIdx.x >> 5]);
 }
 
 // Vertical paths + sum + WTA of an initial-disparity level, G lanes per column. last_base starts
