@@ -173,8 +173,14 @@ void sgm_set_process_error(const char* msg) { set_error(nullptr, "%s", msg); }
 int64_t sgm_float_wait_timeouts();  // float_sgm.cu
 
 // One matching level (the state of one StereoCuda instance).
+constexpr int kModes = 3;  // kernel modes of a matcher, see KernelMode
+
+// Initialised matchers of the process (single-level ones and pyramids, not a pyramid's levels).
+static std::atomic<int> g_live_matchers{0};
+
 struct sgm_engine {
   bool ready = false;
+  bool counted = false;  // in g_live_matchers
   int dev = 0;
   int nsm = 148;  // SMs of the device (set in init)
   int W = 0, H = 0, M = 0, D = 0;
@@ -215,7 +221,9 @@ struct sgm_engine {
   int tune_row_kernel = 0;
   // 0: the default, else 1 plain loads, 2 prefetch ring, 3 u16x2 per column, 4 one warp per column
   int tune_col_kernel = 0;
-  bool latency = false;     // variant 4 in place of the default (see KernelMode)
+  // variant 4 in place of the default (see KernelMode): 1 as set by hand, 2 without the volume that its
+  // column kernels of the 32-disparity levels allocate
+  int latency = 0;
   int tune_row_lanes = 0;   // variant 3: lanes per scanline (0: default)
   int tune_col_lanes = 0;
   bool bt_stored = true;    // the last match wrote the bottom->top volume to global memory
@@ -228,10 +236,10 @@ struct sgm_engine {
   } tmap_key[5];
   // img[0], img[1] -> out captured as a CUDA graph after a first direct run (matches without
   // initial disparities or a right map); later matches copy in, launch it, copy out. One graph
-  // per kernel mode (0: the matcher's tuning, 1: the latency kernels of KernelMode).
-  cudaGraphExec_t gexec[2] = {};
-  int direct_runs[2] = {};
-  int64_t graph_launches[2] = {};
+  // per kernel mode (0: the matcher's tuning, 1 and 2: the latency kernels of KernelMode).
+  cudaGraphExec_t gexec[kModes] = {};
+  int direct_runs[kModes] = {};
+  int64_t graph_launches[kModes] = {};
   cudaEvent_t done = nullptr;  // blocking-sync event of the synchronous host API (see wait_stream)
   // Stages of a match: an NVTX range each, and with print_log a CUDA event at every stage boundary
   // for the per-stage report of the synchronous host API.
@@ -242,7 +250,7 @@ struct sgm_engine {
   cudaEvent_t stage_ev[kMaxStages] = {};
   const char* stage_name[kMaxStages] = {};
   void drop_graph() {
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < kModes; ++k) {
       if (gexec[k]) cudaGraphExecDestroy(gexec[k]);
       gexec[k] = nullptr;
       direct_runs[k] = 0;
@@ -259,6 +267,8 @@ struct sgm_engine {
   int census_bytes() const { return opt.cs_type == 1 ? 8 : 4; }
 
   void free_all() {
+    if (counted) --g_live_matchers;
+    counted = false;
     drop_graph();
     if (done) cudaEventDestroy(done);
     done = nullptr;
@@ -974,6 +984,26 @@ int init4_cols(sgm_engine* e, const int16_t* il, const int16_t* ir, const sgm::I
                         *mc, *mo, il, ir, out, P));
 }
 
+// Top to bottom with the WTA, needing no top-to-bottom volume: for the device API, which allocates
+// nothing. Slower than both column directions beside the row scans and a WTA launch after them (one
+// 3-level pyramid of 1242x375 alone 367 against 331 us, three in flight 207 against 197; 4800x3409
+// 5.75 against 5.32 ms, 4.99 against 4.83): a level stays with those once it holds the volume.
+inline int init4_cols_wta(sgm_engine* e, const int16_t* il, const int16_t* ir, float* wta, const sgm::InitParams& P,
+                          const sgm::WtaParams& Q, cudaStream_t s) {
+  const int nv = e->nviews();
+  const dim3 grid((unsigned)((e->W + kScan4ColWarps - 1) / kScan4ColWarps), nv);
+  const CUtensorMap *mc, *mb, *ml, *mr;
+  int st = volume_map(e, 0, e->cost, nv, &mc);
+  if (!st) st = volume_map(e, 1, e->bt, nv, &mb);
+  if (!st) st = volume_map(e, 2, e->lr, nv, &ml);
+  if (!st) st = volume_map(e, 3, e->rl, nv, &mr);
+  if (st) return st;
+  SGM_CUDA_TRY(e, sgm::prefer_max_shared(sgm::k_vscan_wta_init4<kScan4ColWarps>));
+  return SGM_LAUNCH(e, s, "vpaths_wta_init",
+                    sgm::k_vscan_wta_init4<kScan4ColWarps><<<grid, 32 * kScan4ColWarps, 0, s>>>(
+                        *mc, *mb, *ml, *mr, il, ir, wta, P, Q));
+}
+
 inline int init4_cols_both(sgm_engine* e, const int16_t* il, const int16_t* ir, const sgm::InitParams& P,
                            cudaStream_t s) {
   const int st = init4_cols<1>(e, il, ir, P, s);
@@ -1014,15 +1044,22 @@ int launch_init(sgm_engine* e, const Word* csl, const Word* csr, const int16_t* 
   const bool rows4 = tune_row == 4, cols4 = tune_col == 4;
   // rows reading the cost volume (variants 3 and 4) and columns split into two passes
   auto rows_cv = [&](cudaStream_t ms) { return rows4 ? init4_rows(e, il, ir, P, ms) : init3_rows(e, il, ir, P, ms); };
+  const bool fused = lat && e->latency == 2 && !e->tb;
   auto cols_bt = [&](cudaStream_t ss) {
-    return cols4 ? init4_cols_both(e, il, ir, P, ss) : init3_cols<1>(e, il, ir, wta, P, Q3, ss);
+    return fused   ? init4_cols<1>(e, il, ir, P, ss)
+           : cols4 ? init4_cols_both(e, il, ir, P, ss)
+                   : init3_cols<1>(e, il, ir, wta, P, Q3, ss);
+  };
+  auto cols_wta = [&](cudaStream_t ms) {
+    return fused   ? init4_cols_wta(e, il, ir, wta, P, Q3, ms)
+           : cols4 ? init4_wta(e, il, ir, wta, P, Q3, ms)
+                   : init3_cols<2>(e, il, ir, wta, P, Q3, ms);
   };
   int st;
   if ((rows3 || rows4) && (cols3 || cols4) && kSplitColumns) {  // bottom-to-top pass beside the row scans
     st = init3_cost<Word>(e, csl, csr, il, ir, P, e->stream);
     if (!st) st = fork_join(e, e->stream, cols_bt, rows_cv);
-    if (st) return st;
-    return cols4 ? init4_wta(e, il, ir, wta, P, Q3, e->stream) : init3_cols<2>(e, il, ir, wta, P, Q3, e->stream);
+    return st ? st : cols_wta(e->stream);
   }
   if (rows3 || rows4) {
     st = init3_cost<Word>(e, csl, csr, il, ir, P, e->stream);
@@ -1066,8 +1103,8 @@ int launch_init(sgm_engine* e, const Word* csl, const Word* csr, const int16_t* 
   size_t vsmem = 0;
   if (cols3) return init3_cols<0>(e, il, ir, wta, P, Q3, e->stream);
   if (cols4) {
-    st = init4_cols_both(e, il, ir, P, e->stream);
-    return st ? st : init4_wta(e, il, ir, wta, P, Q3, e->stream);
+    st = cols_bt(e->stream);
+    return st ? st : cols_wta(e->stream);
   }
   if (tune_col != 2) {
     C = e->tune_cols > 0 ? e->tune_cols : 8;
@@ -1363,27 +1400,33 @@ struct HostCall {
   bool (*poll() const)() { return latency() ? few_host_calls : nullptr; }
 };
 
-// Latency kernels on the given engines for the scope of one match, when `latency` and every engine
-// is at the default tuning; mode() is the graph slot to use.
+// Latency kernels (sgm_engine::latency: want, 0 for none) on the given engines for the scope of one
+// match when every engine is at the default tuning; mode() is the graph slot to use.
 struct KernelMode {
   sgm_engine* const* lv;
-  int n;
-  bool on = false;
-  KernelMode(sgm_engine* const* levels, int count, bool latency) : lv(levels), n(count) {
-    if (!latency) return;
+  int n, on = 0;
+  KernelMode(sgm_engine* const* levels, int count, int want) : lv(levels), n(count) {
     for (int i = 0; i < n; ++i)
       if (!lv[i]->tuning_is_default()) return;
-    on = true;
-    for (int i = 0; i < n; ++i) lv[i]->latency = true;
+    on = want;
+    for (int i = 0; i < n; ++i) lv[i]->latency = on;
   }
   ~KernelMode() {
-    if (on)
-      for (int i = 0; i < n; ++i) lv[i]->latency = false;
+    for (int i = 0; i < n; ++i) lv[i]->latency = 0;
   }
   KernelMode(const KernelMode&) = delete;
   KernelMode& operator=(const KernelMode&) = delete;
-  int mode() const { return on ? 1 : 0; }
+  int mode() const { return on; }
 };
+
+// The device API (sgm_match_device, sgm_pyr_match_device) does not wait, so it cannot know how much of
+// its work is in flight. While at most kLatencyInFlight matchers are initialised in the process, no
+// more than that many matches can share the GPU, and the latency kernels are the faster ones at
+// every number of them (us a match with one .. eight matchers in flight on one B200: 450x375, D = 64
+// 110 .. 57, default kernels 414 .. 78; 1242x375, D = 64 220 .. 149, 767 .. 153; 957x541, D = 128
+// 388 .. 293, 1160 .. 303). With 32 matchers the default kernels lead by 3 to 7 % (D = 64, pyramids), so
+// larger pools keep them. Both give the same bits. Nothing is allocated for it (mode 2).
+bool few_matchers() { return g_live_matchers.load(std::memory_order_relaxed) <= kLatencyInFlight; }
 
 int enqueue_depth(sgm_engine* e, const float* disp, float* depth, const sgm_camera_t& c, cudaStream_t s) {
   const int n = (int)e->npix();
@@ -1397,6 +1440,7 @@ int enqueue_depth(sgm_engine* e, const float* disp, float* depth, const sgm_came
 // ------------------------------------------------------------------------------------------
 struct sgm_pyramid {
   bool ready = false;
+  bool counted = false;  // in g_live_matchers
   int W = 0, H = 0, layers = 0;
   std::vector<sgm_engine*> lv;
   std::vector<uint8_t*> imgs_l, imgs_r;  // decimated images per level (level 0 unused)
@@ -1413,13 +1457,13 @@ struct sgm_pyramid {
   float* disp0 = nullptr;  // finest-level disparity in depth mode
   // The whole pyramid (in_l, in_r -> out) captured once as a CUDA graph after a first direct run;
   // later matches copy in, launch it, copy out. One graph per kernel mode (see KernelMode).
-  cudaGraphExec_t gexec[2] = {};
-  int direct_runs[2] = {};
-  int64_t graph_launches[2] = {};  // kernels inside the graph
+  cudaGraphExec_t gexec[kModes] = {};
+  int direct_runs[kModes] = {};
+  int64_t graph_launches[kModes] = {};  // kernels inside the graph
   cudaEvent_t done = nullptr;  // blocking-sync event of the synchronous host API (see wait_stream)
 
   void drop_graph() {
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < kModes; ++k) {
       if (gexec[k]) cudaGraphExecDestroy(gexec[k]);
       gexec[k] = nullptr;
       direct_runs[k] = 0;
@@ -1427,6 +1471,8 @@ struct sgm_pyramid {
   }
 
   void free_all() {
+    if (counted) --g_live_matchers;
+    counted = false;
     drop_graph();
     if (done) cudaEventDestroy(done);
     done = nullptr;
@@ -1570,8 +1616,13 @@ int sgm_init(sgm_handle_t h, int32_t width, int32_t height, int32_t min_disparit
              const sgm_option_t* option, int32_t print_log) {
   if (!h || !option) return SGM_ERR_ARG;
   const int st = engine_init(h, width, height, min_disparity, disp_range, option, print_log != 0);
-  if (st) h->free_all();
-  return st;
+  if (st) {
+    h->free_all();
+    return st;
+  }
+  h->counted = true;
+  ++g_live_matchers;
+  return SGM_OK;
 }
 
 int sgm_set_ext_options(sgm_handle_t h, const sgm_ext_options_t* ext) {
@@ -1649,7 +1700,7 @@ int sgm_match(sgm_handle_t h, const uint8_t* img_left, const uint8_t* img_right,
   const size_t N = h->npix();
   h->launches = 0;
   const HostCall call;
-  const KernelMode km(&h, 1, call.latency());
+  const KernelMode km(&h, 1, call.latency() ? 1 : 0);
   // with print_log: per-stage times, printed like the reference's timers (StereoCudaImpl.cpp:
   // 365-460, 530-543); the match then runs its kernels directly instead of as a graph
   h->stage_timing = h->print_log;
@@ -1707,7 +1758,9 @@ int sgm_match_device(sgm_handle_t h, const uint8_t* d_left, const uint8_t* d_rig
     return SGM_ERR_ARG;
   }
   h->launches = 0;
-  if (!d_init_disp_left && !d_disp_right) return engine_run(h, d_left, d_right, d_disp_left, (cudaStream_t)stream);
+  const KernelMode km(&h, 1, few_matchers() ? 2 : 0);
+  if (!d_init_disp_left && !d_disp_right)
+    return engine_run(h, d_left, d_right, d_disp_left, (cudaStream_t)stream, km.mode());
   return engine_enqueue(h, d_left, d_right, d_init_disp_left, d_disp_left, d_disp_right, (cudaStream_t)stream);
 }
 
@@ -1732,7 +1785,7 @@ int sgm_match2(sgm_handle_t h, const uint8_t* img_left, const uint8_t* img_right
   const size_t N = h->npix();
   h->launches = 0;
   const HostCall call;
-  const KernelMode km(&h, 1, call.latency());
+  const KernelMode km(&h, 1, call.latency() ? 1 : 0);
   SGM_CUDA_TRY(h, cudaMemcpyAsync(h->img[0], img_left, N, cudaMemcpyHostToDevice, h->stream));
   SGM_CUDA_TRY(h, cudaMemcpyAsync(h->img[1], img_right, N, cudaMemcpyHostToDevice, h->stream));
   if (init_disp_left)
@@ -1972,6 +2025,8 @@ int sgm_pyr_init(sgm_pyr_handle_t h, const sgm_pyr_option1_t* o, const sgm_level
     return SGM_ERR_NOMEM;
   }
   h->ready = true;
+  h->counted = true;
+  ++g_live_matchers;
   return SGM_OK;
 }
 
@@ -1982,7 +2037,7 @@ int sgm_pyr_match(sgm_pyr_handle_t h, const uint8_t* img_left, const uint8_t* im
   const size_t N = (size_t)h->W * h->H;
   h->launches = 0;
   const HostCall call;
-  const KernelMode km(h->lv.data(), (int)h->lv.size(), call.latency());
+  const KernelMode km(h->lv.data(), (int)h->lv.size(), call.latency() ? 1 : 0);
   if (cudaMemcpyAsync(h->in_l, img_left, N, cudaMemcpyHostToDevice, h->stream) ||
       cudaMemcpyAsync(h->in_r, img_right, N, cudaMemcpyHostToDevice, h->stream))
     return SGM_ERR_CUDA;
@@ -2002,7 +2057,8 @@ int sgm_pyr_match_device(sgm_pyr_handle_t h, const uint8_t* d_left, const uint8_
   if (!h->ready) return SGM_ERR_STATE;
   if (!d_left || !d_right || !d_disp) return SGM_ERR_ARG;
   h->launches = 0;
-  return pyr_run(h, d_left, d_right, d_disp, stream ? (cudaStream_t)stream : h->stream);
+  const KernelMode km(h->lv.data(), (int)h->lv.size(), few_matchers() ? 2 : 0);
+  return pyr_run(h, d_left, d_right, d_disp, stream ? (cudaStream_t)stream : h->stream, km.mode());
 }
 
 int sgm_pyr_init2(sgm_pyr_handle_t h, const sgm_pyr_option2_t* o, const sgm_level_override_t* ov,

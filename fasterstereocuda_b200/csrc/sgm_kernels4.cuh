@@ -358,16 +358,18 @@ __global__ void __launch_bounds__(32 * WPB)
 // parabola as in wta_pixel; tie rules: kTieRefB200 the lowest tied d whose candidate is valid
 // (every tied lane stores its own result there, a valid one wins), 1 / 2 the highest tied d, 0 / 3
 // the lowest (one disparity per lane: lane order is disparity order). A row is read as two 16-byte
-// words; S(d) is summed in 16-bit halves, its minimum taken by SIMD minima and the tied set kept as
-// a bit mask; S at a candidate's neighbours comes from single bytes.
+// words (unit u at u ^ sw: rows of a swizzled box); S(d) is summed in 16-bit halves, its minimum
+// taken by SIMD minima and the tied set kept as a bit mask; S at a candidate's neighbours comes from
+// single bytes.
 __device__ __forceinline__ float init_wta_rows(const uint8_t* a, const uint8_t* b, const uint8_t* c,
-                                               const uint8_t* e, int base, const WtaParams& Q) {
+                                               const uint8_t* e, int base, const WtaParams& Q, int sw = 0) {
   constexpr int D = kLevelRange;
   uint32_t lo[D / 4], hi[D / 4];  // lo[k] = S(4k) | S(4k + 2) << 16, hi[k] = S(4k + 1) | S(4k + 3) << 16
 #pragma unroll
   for (int q = 0; q < D / 16; ++q) {
-    const uint4 va = reinterpret_cast<const uint4*>(a)[q], vb = reinterpret_cast<const uint4*>(b)[q];
-    const uint4 vc = reinterpret_cast<const uint4*>(c)[q], ve = reinterpret_cast<const uint4*>(e)[q];
+    const int u = q ^ sw;
+    const uint4 va = reinterpret_cast<const uint4*>(a)[u], vb = reinterpret_cast<const uint4*>(b)[u];
+    const uint4 vc = reinterpret_cast<const uint4*>(c)[u], ve = reinterpret_cast<const uint4*>(e)[u];
     const uint32_t wa[4] = {va.x, va.y, va.z, va.w}, wb[4] = {vb.x, vb.y, vb.z, vb.w};
     const uint32_t wc[4] = {vc.x, vc.y, vc.z, vc.w}, we[4] = {ve.x, ve.y, ve.z, ve.w};
 #pragma unroll
@@ -389,7 +391,10 @@ __device__ __forceinline__ float init_wta_rows(const uint8_t* a, const uint8_t* 
     tied |= ((el & 1u) | ((eh & 1u) << 1) | ((el >> 14) & 4u) | ((eh >> 13) & 8u)) << (4 * k);
   }
   const float ut = __fsub_rn(1.0f, Q.uniqueness);
-  auto sum_at = [&](int d) { return (uint32_t)a[d] + b[d] + c[d] + e[d]; };
+  auto sum_at = [&](int d) {
+    const int o = d ^ (sw << 4);
+    return (uint32_t)a[o] + b[o] + c[o] + e[o];
+  };
   auto candidate = [&](int d) {
     if (d <= 1 || d >= Q.dmax_excl) return kInvalidFloat;
     const float c1 = (float)sum_at(d - 1), c2 = (float)m, c3 = (float)sum_at(d + 1);
@@ -431,6 +436,119 @@ __global__ void __launch_bounds__(128) k_wta_init4(const uint8_t* __restrict__ b
     }
   }
   disp[(size_t)view * Q.dstride + (size_t)y * W + x] = dv;
+}
+
+// Top-to-bottom scan of a 32-disparity level with the WTA: as k_vscan_init4 with PASS 3, but a chunk's
+// pixels take their WTA, one lane each, from the chunk's path costs and the boxes of the three stored
+// paths, so the level needs no top-to-bottom volume and moves 4 bytes a voxel where PASS 3 and
+// k_wta_init4 move 6; it can only follow the row scans, where PASS 3 runs beside them.
+template <int WPB>
+__global__ void __launch_bounds__(32 * WPB)
+    k_vscan_wta_init4(const __grid_constant__ CUtensorMap m_cost, const __grid_constant__ CUtensorMap m_bt,
+                      const __grid_constant__ CUtensorMap m_lr, const __grid_constant__ CUtensorMap m_rl,
+                      const int16_t* __restrict__ init_l, const int16_t* __restrict__ init_r,
+                      float* __restrict__ disp, InitParams P, WtaParams Q) {
+  constexpr int D = kLevelRange, C = kScanChunk, BOX = C * D, NB = 3;
+  __shared__ __align__(1024) uint8_t cbuf[WPB][NB + 3][BOX];  // cost; bt, lr, rl
+  __shared__ __align__(8) uint64_t bars[WPB][NB + 1];         // bars[NB]: the stored paths
+  __shared__ __align__(16) uint32_t par[WPB][2][C];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0) {
+    for (int b = 0; b <= NB; ++b) mbar_init(&bars[w][b], 1);
+    mbar_fence_init();
+  }
+  __syncwarp();
+  const int W = P.W, H = P.H;
+  const int x = blockIdx.x * WPB + w, view = blockIdx.y;
+  if (x >= W) return;  // the whole warp
+  disp += (size_t)view * Q.dstride + x;
+  if (x < P.x0) {
+    for (int y = lane; y < H; y += 32) disp[(size_t)y * W] = kInvalidFloat;
+    return;
+  }
+  // the swizzle pattern is a function of the shared address: the boxes must start on 1 KB
+  if (smem_u32(&cbuf[0][0][0]) & 1023u) {
+    if (lane == 0) atomicAdd(&g_scan_wait_timeouts, 1u);
+    return;
+  }
+  const int16_t* ib = (view == 0 ? init_l : init_r) + x;
+  const int nch = (H + C - 1) / C;
+  auto issue_cost = [&](int c) {  // lane 0
+    const int b = c % NB;
+    mbar_expect_tx(&bars[w][b], BOX);
+    tma_load_3d(cbuf[w][b], &m_cost, x * D, C * c, view, &bars[w][b]);
+  };
+  auto issue_paths = [&](int c) {  // lane 0
+    mbar_expect_tx(&bars[w][NB], 3 * BOX);
+    tma_load_3d(cbuf[w][NB + 0], &m_bt, x * D, C * c, view, &bars[w][NB]);
+    tma_load_3d(cbuf[w][NB + 1], &m_lr, x * D, C * c, view, &bars[w][NB]);
+    tma_load_3d(cbuf[w][NB + 2], &m_rl, x * D, C * c, view, &bars[w][NB]);
+  };
+  auto base_of = [&](int c) {
+    const int y = C * c + lane;
+    return y < H ? (int)ib[(size_t)y * W] : (int)kInvalidShort;
+  };
+  if (lane == 0) {
+    issue_cost(0);
+    if (nch > 1) issue_cost(1);
+    issue_paths(0);
+  }
+  const bool col_ok = x >= Q.xlo && x <= Q.xhi;
+  uint32_t phase = 0u;  // bit b: parity of buffer b's next phase
+  ChunkState st{(int)ib[0], false};  // row 0's base
+  int bnext = base_of(0);
+  uint32_t L = 0;
+  const int lo0 = lane, lo1 = lane ^ 16;  // this lane's byte of a box row under the two swizzles
+  for (int c = 0; c < nch; ++c) {
+    const int b = c % NB;
+    const int bcur = bnext;
+    if (c + 1 < nch) bnext = base_of(c + 1);
+    uint32_t flags, p2;
+    chunk_params(bcur, c * C, min(C, H - c * C), false, P, st, flags, p2);
+    par[w][0][lane] = flags;
+    par[w][1][lane] = p2;
+    if (!mbar_wait_warp(&bars[w][b], (phase >> b) & 1u)) {
+      scan_give_up_mask(bars[w], phase, (1u << NB) | (1u << b) | (c + 1 < nch ? 1u << ((c + 1) % NB) : 0u));
+      return;
+    }
+    phase ^= 1u << b;
+    __syncwarp();
+    uint8_t* box = cbuf[w][b];
+    auto at = [&](int j) { return box + j * D + (box_sw<D>(j) ? lo1 : lo0); };
+    uint32_t fl[C], pp[C], cvr[C];
+#pragma unroll
+    for (int j = 0; j < C; ++j) {
+      fl[j] = par[w][0][j];
+      pp[j] = par[w][1][j];
+      cvr[j] = *at(j);
+    }
+#pragma unroll
+    for (int j = 0; j < C; ++j) {
+      if (c == 0 && j == 0) L = cvr[0];
+      else scan_step(L, cvr[j], fl[j], pp[j], P.p1);
+      *at(j) = (uint8_t)L;
+    }
+    __syncwarp();  // the chunk's path costs, written by disparity, are read by pixel
+    if (!mbar_wait_warp(&bars[w][NB], (phase >> NB) & 1u)) {
+      scan_give_up_mask(bars[w], phase, (1u << NB) | (c + 1 < nch ? 1u << ((c + 1) % NB) : 0u));
+      return;
+    }
+    phase ^= 1u << NB;
+    const int y = C * c + lane, o = lane * D;
+    if (y < H) {
+      float dv = kInvalidFloat;
+      if (col_ok && y >= Q.ylo && y <= Q.yhi && y < Q.rows && bcur != kInvalidShort)
+        dv = init_wta_rows(box + o, cbuf[w][NB] + o, cbuf[w][NB + 1] + o, cbuf[w][NB + 2] + o, bcur, Q,
+                           box_sw<D>(lane));
+      disp[(size_t)y * W] = dv;
+    }
+    fence_proxy_async();  // the accesses of the boxes before the copies that refill them
+    __syncwarp();
+    if (lane == 0) {
+      if (c + 1 < nch) issue_paths(c + 1);
+      if (c + 2 < nch) issue_cost(c + 2);
+    }
+  }
 }
 
 }  // namespace sgm

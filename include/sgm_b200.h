@@ -98,7 +98,9 @@ SGM_API int sgm_get_ext_options(sgm_handle_t h, sgm_ext_options_t* ext);
  * them (every variant is bit-exact), only speed does. 0 everywhere = defaults; a matcher left at
  * the defaults runs, in the synchronous host API (sgm_match, sgm_match2, sgm_pyr_match,
  * sgm_pyr_match2), row_kernel = col_kernel = 4 while at most eight such calls are in flight in
- * the process (a few callers matching one frame at a time) and the defaults below otherwise.
+ * the process (a few callers matching one frame at a time) and the defaults below otherwise; in the
+ * device API (sgm_match_device, sgm_pyr_match_device) while at most eight matchers are initialised
+ * in the process (without the extra volume of column variant 4: nothing is allocated there).
  * While at most eight calls are in flight they also wait for their results by polling; beyond
  * that they sleep on a blocking-sync event. */
 typedef struct sgm_tuning_t {
