@@ -38,19 +38,24 @@ __device__ __forceinline__ void bulk_to_smem(void* dst, const void* src, uint32_
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
-// Waits for the phase of bar with the given parity; false after g_wait_limit polls.
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// Waits for the phase of bar with the given parity; false after g_wait_limit polls. The limit is read
+// only once a first poll has failed: chunks are copied ahead, so most waits end at the first poll, and
+// the load of the limit was most of their ~350 cycles (a chunk of 32 steps takes ~3000).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t a = smem_u32(bar);
+  if (mbar_try_wait(a, parity)) return true;
   const unsigned int limit = g_wait_limit;
-  for (unsigned int it = 0; it < limit; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
+  for (unsigned int it = 1; it < limit; ++it)
+    if (mbar_try_wait(a, parity)) return true;
   return false;
 }
 // The same wait by every lane of the warp, with one verdict for all: the warp stays converged for
