@@ -47,8 +47,10 @@ struct ChunkState {
 // b: this lane's step base (INVALID for lanes past the chunk); gs0: global index of the chunk's
 // first step; n: steps in the chunk; first_sets_base: the scanline's first pixel sets last_base
 // (horizontal scans) or keeps the one given (vertical scans, cusgm_ca.cu:1291).
+// p2tab: P2' by k = |last_base - base + 1| (fill_p2_table), in shared memory: the divisions are the
+// longest part of a chunk's parameters.
 __device__ __forceinline__ void chunk_params(int b, int gs0, int n, bool first_sets_base, const InitParams& P,
-                                             ChunkState& st, uint32_t& flags, uint32_t& p2) {
+                                             const uint32_t* p2tab, ChunkState& st, uint32_t& flags, uint32_t& p2) {
   const int j = threadIdx.x & 31;
   const bool in = j < n;
   const bool first = gs0 + j == 0;
@@ -60,9 +62,7 @@ __device__ __forceinline__ void chunk_params(int b, int gs0, int n, bool first_s
   const int lb = prev ? from_prev : st.carry_base;
   const int s = b - lb;
   const int sc = s < -64 ? -64 : (s > 64 ? 64 : s);
-  const int k = abs(lb - b + 1);
-  const int32_t q = k ? P.p2s / k : P.p2_div0;
-  p2 = (uint32_t)(P.p1s > q ? P.p1s : q);
+  p2 = step_valid ? p2_term(p2tab, abs(lb - b + 1), P) : 0u;
   // the previous step was skipped: the chunk's carry for lane 0, the left neighbour's flag else
   const unsigned inv = __ballot_sync(kFull, in && !first && b == kInvalidShort);
   const bool prev_inv = j == 0 ? st.carry_invalid : ((inv >> (j - 1)) & 1u);
@@ -124,13 +124,15 @@ __global__ void __launch_bounds__(32 * WPB) k_hscan_init4(const uint8_t* __restr
   constexpr int D = kLevelRange, C = kScanChunk, NB = 2;
   __shared__ __align__(128) uint8_t cbuf[WPB][NB][C * D];
   __shared__ __align__(8) uint64_t bars[WPB][NB];
-  __shared__ uint32_t par[WPB][C];
+  __shared__ __align__(16) uint32_t par[WPB][C];
+  __shared__ uint32_t p2tab[kP2Tab];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) {
     for (int b = 0; b < NB; ++b) mbar_init(&bars[w][b], 1);
     mbar_fence_init();
   }
-  __syncwarp();
+  fill_p2_table(p2tab, P, threadIdx.x, 32 * WPB);
+  __syncthreads();
   const int H = P.H, W = P.W;
   const int i = blockIdx.x * WPB + w;
   if (i >= nviews * 2 * H) return;  // the whole warp
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(32 * WPB) k_hscan_init4(const uint8_t* __restr
   // packed step parameters of chunk c (lane j: step j) and whether it takes the fast path
   auto params = [&](int c, int bse, uint32_t& pk, bool& fast) {
     uint32_t flags, p2;
-    chunk_params(bse, c * C, chunk_n(c), true, P, st, flags, p2);
+    chunk_params(bse, c * C, chunk_n(c), true, P, p2tab, st, flags, p2);
     pk = (p2 << 10) | flags;
     fast = __all_sync(kFull, (flags & (kStepValid | kPrevInvalid)) == kStepValid || (c == 0 && lane == 0));
   };
@@ -250,12 +252,14 @@ __global__ void __launch_bounds__(32 * WPB)
   __shared__ __align__(1024) uint8_t cbuf[WPB][NB][BOX];
   __shared__ __align__(8) uint64_t bars[WPB][NB];
   __shared__ __align__(16) uint32_t par[WPB][2][C];
+  __shared__ uint32_t p2tab[kP2Tab];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) {
     for (int b = 0; b < NB; ++b) mbar_init(&bars[w][b], 1);
     mbar_fence_init();
   }
-  __syncwarp();
+  fill_p2_table(p2tab, P, threadIdx.x, 32 * WPB);
+  __syncthreads();
   const int W = P.W, H = P.H;
   const int x = blockIdx.x * WPB + w;
   const int view = blockIdx.y;
@@ -293,7 +297,7 @@ __global__ void __launch_bounds__(32 * WPB)
     const int bcur = bnext;
     if (c + 1 < nch) bnext = base_of(c + 1);
     uint32_t flags, p2;
-    chunk_params(bcur, c * C, n, false, P, st, flags, p2);
+    chunk_params(bcur, c * C, n, false, P, p2tab, st, flags, p2);
     par[w][0][lane] = flags;
     par[w][1][lane] = p2;
     if (!mbar_wait_warp(&bars[w][b], (phase >> b) & 1u)) {
@@ -452,12 +456,14 @@ __global__ void __launch_bounds__(32 * WPB)
   __shared__ __align__(1024) uint8_t cbuf[WPB][NB + 3][BOX];  // cost; bt, lr, rl
   __shared__ __align__(8) uint64_t bars[WPB][NB + 1];         // bars[NB]: the stored paths
   __shared__ __align__(16) uint32_t par[WPB][2][C];
+  __shared__ uint32_t p2tab[kP2Tab];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) {
     for (int b = 0; b <= NB; ++b) mbar_init(&bars[w][b], 1);
     mbar_fence_init();
   }
-  __syncwarp();
+  fill_p2_table(p2tab, P, threadIdx.x, 32 * WPB);
+  __syncthreads();
   const int W = P.W, H = P.H;
   const int x = blockIdx.x * WPB + w, view = blockIdx.y;
   if (x >= W) return;  // the whole warp
@@ -504,7 +510,7 @@ __global__ void __launch_bounds__(32 * WPB)
     const int bcur = bnext;
     if (c + 1 < nch) bnext = base_of(c + 1);
     uint32_t flags, p2;
-    chunk_params(bcur, c * C, min(C, H - c * C), false, P, st, flags, p2);
+    chunk_params(bcur, c * C, min(C, H - c * C), false, P, p2tab, st, flags, p2);
     par[w][0][lane] = flags;
     par[w][1][lane] = p2;
     if (!mbar_wait_warp(&bars[w][b], (phase >> b) & 1u)) {
