@@ -779,8 +779,7 @@ int forward_impl(const float* cost, const float* p1, const float* p2, int B, int
   int st = cost_map(cost, B, H, W, D, &tm);
   if (st) return st;
   constexpr size_t smem = fwd_smem_bytes<K>();
-  if (cudaFuncSetAttribute(k_float_fwd<K, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return check("float forward attribute");
+  static_assert(smem <= 48 * 1024, "no opt-in for more shared memory needed");
   k_float_fwd<K, REC><<<a.q.first_block[4], kWarps * 32, smem, s>>>(tm, a);
   st = check("float forward");
   if (st) return st;

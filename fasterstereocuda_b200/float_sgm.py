@@ -7,6 +7,7 @@ finite-difference reference.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 
 import torch
 
@@ -38,7 +39,21 @@ def _aligned(t):
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
+@functools.lru_cache(maxsize=64)
+def _elems(B, H, W, D):
+    """(volume, records, workspace) sizes in floats, each a multiple of 16 bytes"""
+    lib = _lib()
+    return B * H * W * D, lib.sgm_float_checkpoint_elems(B, H, W, D), lib.sgm_float_workspace_elems(B, H, W, D)
+
+
+def _check(lib, status, what):
+    if status != 0:
+        raise RuntimeError(f"float SGM {what} failed: {lib.sgm_last_error(None).decode()}")
+
+
 class FloatSGM(torch.autograd.Function):
+    # A 64x48 crop's forward and backward are ~40 us of kernels: the host's share is kept small with
+    # one allocation for what the backward pass needs and one for each pass's scratch.
     @staticmethod
     def forward(ctx, cost, p1, p2, temperature=1.0, grad_enabled=True):
         if not (cost.is_cuda and cost.dtype == torch.float32 and cost.dim() == 4):
@@ -46,42 +61,37 @@ class FloatSGM(torch.autograd.Function):
         cost, p1, p2 = _aligned(cost.contiguous()), p1.contiguous().float(), p2.contiguous().float()
         B, H, W, D = cost.shape
         lib = _lib()
-        sum_ = torch.empty_like(cost)
-        work = torch.empty(lib.sgm_float_workspace_elems(B, H, W, D), dtype=torch.float32, device=cost.device)
-        disp = torch.empty((B, H, W), dtype=torch.float32, device=cost.device)
-        stream = torch.cuda.current_stream(cost.device).cuda_stream
-        if not (grad_enabled and any(ctx.needs_input_grad)):  # no backward pass: nothing to keep for it
-            st = lib.sgm_float_disparity(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D,
-                                         float(temperature), sum_.data_ptr(), work.data_ptr(), disp.data_ptr(), stream)
-            if st != 0:
-                raise RuntimeError(f"float SGM forward failed: {lib.sgm_last_error(None).decode()}")
+        vol, rec, scratch = _elems(B, H, W, D)
+        dev, temperature = cost.device, float(temperature)
+        keep = grad_enabled and any(ctx.needs_input_grad)  # else no backward pass: nothing is kept for it
+        kept = torch.empty(vol + rec if keep else vol, dtype=torch.float32, device=dev)  # S, then the records
+        work = torch.empty(scratch, dtype=torch.float32, device=dev)
+        disp = torch.empty((B, H, W), dtype=torch.float32, device=dev)
+        sum_, stream = kept.data_ptr(), torch.cuda.current_stream(dev).cuda_stream
+        if not keep:
+            _check(lib, lib.sgm_float_disparity(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D, temperature,
+                                                sum_, work.data_ptr(), disp.data_ptr(), stream), "forward")
             return disp
-        ckpt = torch.empty(lib.sgm_float_checkpoint_elems(B, H, W, D), dtype=torch.float32, device=cost.device)
-        st = lib.sgm_float_forward(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D, float(temperature),
-                                   sum_.data_ptr(), ckpt.data_ptr(), work.data_ptr(), disp.data_ptr(), stream)
-        if st != 0:
-            raise RuntimeError(f"float SGM forward failed: {lib.sgm_last_error(None).decode()}")
-        ctx.save_for_backward(cost, p1, p2, sum_, ckpt)
-        ctx.temperature = float(temperature)
+        _check(lib, lib.sgm_float_forward(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D, temperature,
+                                          sum_, sum_ + 4 * vol, work.data_ptr(), disp.data_ptr(), stream), "forward")
+        ctx.save_for_backward(cost, p1, p2, kept)
+        ctx.temperature = temperature
         return disp
 
     @staticmethod
     def backward(ctx, grad_disp):
-        cost, p1, p2, sum_, ckpt = ctx.saved_tensors
+        cost, p1, p2, kept = ctx.saved_tensors
         B, H, W, D = cost.shape
         lib = _lib()
+        vol, _, scratch = _elems(B, H, W, D)
         g = grad_disp.contiguous().float()
-        gsum = torch.empty_like(cost)
-        gcost = torch.empty_like(cost)
-        gp1 = torch.empty_like(p1)
-        gp2 = torch.empty_like(p2)
-        work = torch.empty(lib.sgm_float_workspace_elems(B, H, W, D), dtype=torch.float32, device=cost.device)
-        st = lib.sgm_float_backward(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D, ctx.temperature,
-                                    sum_.data_ptr(), ckpt.data_ptr(), g.data_ptr(), gsum.data_ptr(),
-                                    work.data_ptr(), gcost.data_ptr(), gp1.data_ptr(), gp2.data_ptr(),
-                                    torch.cuda.current_stream(cost.device).cuda_stream)
-        if st != 0:
-            raise RuntimeError(f"float SGM backward failed: {lib.sgm_last_error(None).decode()}")
+        work = torch.empty(vol + scratch, dtype=torch.float32, device=cost.device)  # gradient of S, workspace
+        gcost, gp1, gp2 = torch.empty_like(cost), torch.empty_like(p1), torch.empty_like(p2)
+        sum_, gsum = kept.data_ptr(), work.data_ptr()
+        _check(lib, lib.sgm_float_backward(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D, ctx.temperature,
+                                           sum_, sum_ + 4 * vol, g.data_ptr(), gsum, gsum + 4 * vol,
+                                           gcost.data_ptr(), gp1.data_ptr(), gp2.data_ptr(),
+                                           torch.cuda.current_stream(cost.device).cuda_stream), "backward")
         return gcost, gp1, gp2, None, None
 
 
