@@ -25,10 +25,10 @@
 // the adjoint routes the gradient of every L_p(d) to C_p(d), to P1(p) or P2(p) and to L_q by them.
 // Storing path states every 8 pixels and repeating the recurrence in the backward read the cost
 // volume a second time and ran the longer half of the backward's chain: 4 x 1242x375 x 64, scan
-// 1576 -> 772 us, with the recording forward scan at 640 us (645 before it).
-// Mapping, backward: a scanline is held by G lanes of a warp, 8 disparities per lane (8 lanes at
-// D = 64), sums by butterflies; the gradient of S is loaded kBwdPF steps ahead. Bound by DRAM:
-// 3.93 GB at 5.1 TB/s at that size.
+// 1576 -> 772 us (eight lanes a line then), with the recording forward scan at 640 us (645 before it).
+// Mapping, backward: a scanline is held by G lanes of a warp, kBwdK disparities per lane (16 lanes at
+// D = 64), sums by butterflies; the gradient of S is copied kBwdPF - 1 steps ahead. At that size
+// 3.93 GB in 735 us, 5.3 TB/s; one image alone is bound by its row steps (~270 ns each).
 //
 // Layouts: cost/sum/grad volumes float [B][H][W][D] (16-byte aligned); maps float [B][H][W];
 // records in four slabs of ckpt, one per path. Paths: 0 top->bottom, 1 left->right,
@@ -51,12 +51,10 @@ namespace {
 constexpr unsigned kFullMask = 0xFFFFFFFFu;
 constexpr int kK = 8;       // disparities per lane of the soft-argmin kernels
 constexpr int kSeg = 8;     // positions per segment of recorded choices
-constexpr int kBwdPF = 4;   // steps that the backward scans load ahead (divides kSeg)
+constexpr int kBwdK = 4;    // disparities per lane of the backward scans
+constexpr int kBwdPF = 8;   // slots of the backward scans' copies ahead (divides kSeg)
 constexpr int kWarps = 4;   // warps per block of the scan kernels
 constexpr int kFC = 16;     // steps per staged chunk of the forward scans (a multiple of kSeg)
-// lanes per scanline of the backward scans at D = 64 and D = 32 (any choice gives the same path
-// states: the per-disparity arithmetic and the exact minimum do not depend on it)
-constexpr int kBwdLanes64 = 8, kBwdLanes32 = 4;
 #define kInf __int_as_float(0x7f800000)
 
 struct Geo {
@@ -487,7 +485,7 @@ struct BwdArgs {
   Grid4 q;
 };
 
-// Codes of the lane's K = 8 disparities over one segment: four words; the two bits of voxel t in slot j.
+// Codes of the lane's K disparities over one segment: K / 2 words; the two bits of voxel t in slot j.
 template <int FK>
 __device__ __forceinline__ constexpr int code_shift(int t, int j) {
   return FK == 2 ? 4 * j + 2 * (t & 1) : 16 * (t & 1) + 2 * j;
@@ -515,10 +513,17 @@ __device__ __forceinline__ void reduce_segment(float (&v)[2 * kSeg], int gl) {
 // arrives at L_p from its successor to the one of S, writes it (the gradient of C_p) and routes it to
 // the predecessor by the recorded choices: gv goes to L_q(d), L_q(d-1), L_q(d+1) or to m_q, and
 // subtracting m_q takes the sum of all that did not jump from L_q(argmin).
-template <int G, int K>
+//
+// The gradient of S arrives kBwdPF - 1 steps ahead by asynchronous copies (cp.async, one group a step):
+// a warp's lanes copy the step's 512 bytes in 16-byte units side by side and read their own unit after a
+// warp barrier. As a ring of registers the loads shared scoreboards with younger loads and with the
+// step's shuffles, and a row step took ~750 cycles.
+// Four disparities per lane: with eight, twice the lines fit a warp, but a step is twice the
+// instructions for one warp to issue, and the row scans take as long as their steps do (one 1242x375
+// image, D = 64, backward pass 581 -> 479 us; four 1294 -> 1274 us, and at D = 32 803 -> 722 us).
+template <int G>
 __global__ void __launch_bounds__(kWarps * 32, 4) k_float_bwd(const BwdArgs a) {
-  static_assert(K == 8, "four words of codes per lane and segment");
-  constexpr int D = G * K, FK = D / 32, PF = kBwdPF;
+  constexpr int K = kBwdK, D = G * K, FK = D / 32, PF = kBwdPF;
   Line ln;
   Geo g;
   if (!locate<G>(a.q, ln, g)) return;
@@ -528,11 +533,14 @@ __global__ void __launch_bounds__(kWarps * 32, 4) k_float_bwd(const BwdArgs a) {
   const bool down = ln.dir < 2;  // paths of ascending position are walked downwards
   const int len = g.len, nseg = g.nseg;
   const long long sd = step * D;
-  const float* gs = a.gsum + base * D + gl * K;
+  static_assert(K == 4, "a unit of 16 bytes a lane and step");
+  __shared__ __align__(16) float4 ring[kWarps][PF][32];
+  float4(*rows)[32] = ring[threadIdx.x >> 5];
+  const float* gs = a.gsum + base * D + gl * K;  // this lane's unit of a step
   float* go = a.gout[ln.dir] + base * D + gl * K;
   float* gp1 = a.gp1[ln.dir];
   float* gp2 = a.gp2[ln.dir];
-  const uint4* codes = reinterpret_cast<const uint4*>(reinterpret_cast<const CodeWord<FK>*>(a.rec[ln.dir]) +
+  const uint2* codes = reinterpret_cast<const uint2*>(reinterpret_cast<const CodeWord<FK>*>(a.rec[ln.dir]) +
                                                       (size_t)ln.line * nseg * 32) + gl;
   const uint2* args = reinterpret_cast<const uint2*>(reinterpret_cast<const char*>(a.rec[ln.dir]) +
                                                      code_bytes<FK>(g.lines, nseg)) + (size_t)ln.line * nseg;
@@ -540,36 +548,49 @@ __global__ void __launch_bounds__(kWarps * 32, 4) k_float_bwd(const BwdArgs a) {
   float gn[K];  // gradient arriving from the successor
 #pragma unroll
   for (int t = 0; t < K; ++t) gn[t] = 0.f;
-  float ring[PF][K];
   auto segment = [&](int si) { return down ? nseg - 1 - si : si; };
   auto position = [&](int seg, int slot) { return seg * kSeg + (down ? kSeg - 1 - slot : slot); };
-  auto fetch = [&](int r, int si, int slot) {  // gradient of S at a slot; nothing past the line
-    if (si >= nseg) return;
-    const int pos = position(segment(si), slot);
-    if (pos < len) loadK<K>(gs + pos * sd, ring[r]);
+  // gradient of S at a slot of segment si into ring row r; nothing past the line; a group either way
+  auto fetch = [&](int r, int si, int slot) {
+    if (si < nseg) {
+      const int pos = position(segment(si), slot);
+      if (pos < len) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sgm::smem_u32(rows[r] + lane)), "l"(gs + pos * sd)
+                     : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // before slot j of segment si: its row is there for every lane; the row of the slot before is refilled
+  auto turn = [&](int si, int j) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PF - 2) : "memory");
+    __syncwarp();
+    const int ahead = j + PF - 1;
+    fetch(ahead % PF, ahead < kSeg ? si : si + 1, ahead % kSeg);
   };
 #pragma unroll
-  for (int j = 0; j < PF; ++j) fetch(j, 0, j);
-  uint4 cw = __ldg(codes + (size_t)segment(0) * G);
+  for (int j = 0; j < PF - 1; ++j) fetch(j, 0, j);
+  uint2 cw = __ldg(codes + (size_t)segment(0) * G);
   uint2 aw = __ldg(args + segment(0));
   for (int si = 0; si < nseg; ++si) {
     const int seg = segment(si);
-    const uint32_t w[4] = {cw.x, cw.y, cw.z, cw.w}, ar[2] = {aw.x, aw.y};
+    const uint32_t w[K / 2] = {cw.x, cw.y}, ar[2] = {aw.x, aw.y};
     if (si + 1 < nseg) {
       cw = __ldg(codes + (size_t)segment(si + 1) * G);
       aw = __ldg(args + segment(si + 1));
     }
     float part[2 * kSeg];  // this lane's share of the P1 and P2 gradients of each slot
     auto step_at = [&](int j, bool start) {
+      turn(si, j);
       const long long off = position(seg, j) * sd;
       float gv[K];
-#pragma unroll
-      for (int t = 0; t < K; t += 2) {
-        const float2 x = __fadd2_rn(make_float2(ring[j % PF][t], ring[j % PF][t + 1]), make_float2(gn[t], gn[t + 1]));
-        gv[t] = x.x;
-        gv[t + 1] = x.y;
-      }
-      fetch(j % PF, j + PF < kSeg ? si : si + 1, (j + PF) % kSeg);
+      const float4 x = rows[j % PF][lane];
+      const float2 lo = __fadd2_rn(make_float2(x.x, x.y), make_float2(gn[0], gn[1]));
+      const float2 hi = __fadd2_rn(make_float2(x.z, x.w), make_float2(gn[2], gn[3]));
+      gv[0] = lo.x;
+      gv[1] = lo.y;
+      gv[2] = hi.x;
+      gv[3] = hi.y;
       if (live) storeK<K>(go + off, gv);
       part[2 * j] = part[2 * j + 1] = 0.f;
       if (start) return;  // the path's first pixel: nothing before it
@@ -622,16 +643,21 @@ __global__ void __launch_bounds__(kWarps * 32, 4) k_float_bwd(const BwdArgs a) {
         if (position(seg, j) < len)
           step_at(j, j == start);
         else
-          fetch(j % PF, j + PF < kSeg ? si : si + 1, (j + PF) % kSeg);
+          turn(si, j);
       }
     }
     reduce_segment<G>(part, gl);
+    if constexpr (G == 2 * kSeg) {  // one value a lane
+      const int pos = position(seg, gl / 2);
+      if (live && pos < len) (gl & 1 ? gp2 : gp1)[base + pos * step] = part[0];
+    } else {
 #pragma unroll
-    for (int i = 0; i < kSeg / G; ++i) {
-      const int pos = position(seg, gl * (kSeg / G) + i);
-      if (live && pos < len) {
-        gp1[base + pos * step] = part[2 * i];
-        gp2[base + pos * step] = part[2 * i + 1];
+      for (int i = 0; i < kSeg / G; ++i) {
+        const int pos = position(seg, gl * (kSeg / G) + i);
+        if (live && pos < len) {
+          gp1[base + pos * step] = part[2 * i];
+          gp2[base + pos * step] = part[2 * i + 1];
+        }
       }
     }
   }
@@ -790,11 +816,11 @@ int forward_impl(const float* cost, const float* p1, const float* p2, int B, int
   return check("soft argmin");
 }
 
-template <int G, int K>
+template <int G>
 int backward_impl(const float* cost, const float* p1, const float* p2, int B, int H, int W, float inv_t,
                   const float* sum, const float* ckpt, const float* grad_disp, float* grad_sum, float* work,
                   float* grad_cost, float* grad_p1, float* grad_p2, cudaStream_t s) {
-  constexpr int D = G * K;
+  constexpr int D = G * kBwdK;
   const size_t V = (size_t)B * H * W * D, npix = (size_t)B * H * W;
   constexpr int GS = D / kK;  // lanes per pixel of the soft-argmin kernels
   const size_t px_per_block = 8 * (32 / GS);
@@ -813,7 +839,7 @@ int backward_impl(const float* cost, const float* p1, const float* p2, int B, in
     a.gp2[i] = maps + (4 + i) * npix;
   }
   a.q = make_grid<G>(B, H, W, D);
-  k_float_bwd<G, K><<<a.q.first_block[4], kWarps * 32, 0, s>>>(a);
+  k_float_bwd<G><<<a.q.first_block[4], kWarps * 32, 0, s>>>(a);
   if ((st = check("float backward"))) return st;
   SumArgs r;
   r.g0 = reinterpret_cast<float4*>(grad_cost);
@@ -891,10 +917,10 @@ int sgm_float_backward(const float* cost, const float* p1, const float* p2, int3
     return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const float inv_t = 1.0f / temperature;
-  return D == 64 ? backward_impl<kBwdLanes64, 64 / kBwdLanes64>(cost, p1, p2, B, H, W, inv_t, sum, ckpt, grad_disp,
-                                                                grad_sum, work, grad_cost, grad_p1, grad_p2, s)
-                 : backward_impl<kBwdLanes32, 32 / kBwdLanes32>(cost, p1, p2, B, H, W, inv_t, sum, ckpt, grad_disp,
-                                                                grad_sum, work, grad_cost, grad_p1, grad_p2, s);
+  return D == 64 ? backward_impl<64 / kBwdK>(cost, p1, p2, B, H, W, inv_t, sum, ckpt, grad_disp, grad_sum, work,
+                                             grad_cost, grad_p1, grad_p2, s)
+                 : backward_impl<32 / kBwdK>(cost, p1, p2, B, H, W, inv_t, sum, ckpt, grad_disp, grad_sum, work,
+                                             grad_cost, grad_p1, grad_p2, s);
 }
 
 }  // extern "C"
