@@ -105,26 +105,33 @@ __device__ __forceinline__ void scan_step_fast(uint32_t& L, uint32_t c, int s, u
 
 // ---------------------------------------------------------------------------------------------
 // Horizontal scans: warp w of the grid owns scanline i = (view, dir, y) as in hpaths3_lane. A
-// chunk is 32 consecutive pixels of the row, one contiguous bulk copy (double-buffered); its
-// costs go to registers at once, which frees the buffer for the chunk after next. Right-to-left
-// scans place a short (last) chunk at the end of the buffer, so that step j of every chunk reads
-// row 31 - j; every chunk runs all 32 steps (the steps past a short chunk are marked skipped and
-// keep the state). Each step stores its 32 path costs straight to global memory (one 32-byte
-// segment per warp). The step parameters of the next chunk are computed
-// beside the steps of this one (they do not depend on the path costs), and a chunk whose steps
-// all have valid bases (the usual case) runs scan_step_fast. Step parameters: kStepValid,
-// kPrevInvalid and the shift in bits 0-9, P2' above them (P1, P2 < 2^22).
+// chunk is 32 consecutive pixels of the row, one contiguous bulk copy (double-buffered).
+// Right-to-left scans place a short (last) chunk at the end of the buffer, so that step j of every
+// chunk reads row 31 - j; every chunk runs all 32 steps (the steps past a short chunk are marked
+// skipped and keep the state). Each step stores its 32 path costs straight to global memory (one
+// 32-byte segment per warp). The step parameters of the next chunk are computed beside the steps
+// of this one (they do not depend on the path costs), and a chunk whose steps all have valid bases
+// (the usual case) runs scan_step_fast. Step parameters: the shift (fast chunks) or kStepValid,
+// kPrevInvalid and the shift in bits 0-9; P2'.
+// A large level is bound by its integer operations (half rate: selects, compares, minima), then by
+// how many warps are there to issue them. So the two directions are separate code (constant
+// offsets), the parameters arrive ready to use, and a step's costs and parameters are read from
+// shared memory kGroup4 steps ahead, not a chunk (152 -> 96 registers, 12 -> 20 warps an SM; 80
+// registers spill): 4800x3409 pyramid, three levels of row scans 2432 -> 1990 us beside the
+// bottom-to-top columns.
 // ---------------------------------------------------------------------------------------------
+constexpr int kGroup4 = 8;
+
 template <int WPB>
-__global__ void __launch_bounds__(32 * WPB) k_hscan_init4(const uint8_t* __restrict__ cost,
+__global__ void __launch_bounds__(32 * WPB, 1) k_hscan_init4(const uint8_t* __restrict__ cost,
                                                           const int16_t* __restrict__ init_l,
                                                           const int16_t* __restrict__ init_r,
                                                           uint8_t* __restrict__ lr, uint8_t* __restrict__ rl,
                                                           InitParams P, int nviews) {
-  constexpr int D = kLevelRange, C = kScanChunk, NB = 2;
+  constexpr int D = kLevelRange, C = kScanChunk, NB = 2, R = kGroup4;
   __shared__ __align__(128) uint8_t cbuf[WPB][NB][C * D];
   __shared__ __align__(8) uint64_t bars[WPB][NB];
-  __shared__ __align__(16) uint32_t par[WPB][C];
+  __shared__ __align__(16) uint2 par[WPB][2][C];
   __shared__ uint32_t p2tab[kP2Tab];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) {
@@ -137,95 +144,162 @@ __global__ void __launch_bounds__(32 * WPB) k_hscan_init4(const uint8_t* __restr
   const int i = blockIdx.x * WPB + w;
   if (i >= nviews * 2 * H) return;  // the whole warp
   const int grp = i / H, y = i - grp * H;
-  const int view = grp >> 1, dir = grp & 1;
+  const int view = grp >> 1;
   const int len = W - P.x0;
   if (len <= 0) return;
   const size_t ro = (size_t)view * P.vstride + (size_t)y * W * D;
   const uint8_t* crow = cost + ro;
-  uint8_t* orow = (dir == 0 ? lr : rl) + ro;
   const int16_t* ib = (view == 0 ? init_l : init_r) + (size_t)y * W;
   const int nch = (len + C - 1) / C;
-  // chunk c: steps [c*C, c*C + n), pixels [chunk_x, chunk_x + n) in memory order (n <= 0: none)
-  auto chunk_n = [&](int c) { return min(C, len - c * C); };
-  auto chunk_x = [&](int c) { return dir == 0 ? P.x0 + c * C : W - (c * C + chunk_n(c)); };
-  auto chunk_off = [&](int c) { return dir == 0 ? 0 : (C - chunk_n(c)) * D; };  // bytes into the buffer
-  auto issue = [&](int c) {  // lane 0
-    const int b = c % NB;
-    const uint32_t bytes = (uint32_t)chunk_n(c) * D;
-    mbar_expect_tx(&bars[w][b], bytes);
-    bulk_to_smem(cbuf[w][b] + chunk_off(c), crow + (size_t)chunk_x(c) * D, bytes, &bars[w][b]);
+  auto scan = [&](auto right_to_left) {
+    constexpr bool kLeft = decltype(right_to_left)::value;
+    constexpr int r0 = kLeft ? (C - 1) * D : 0, dr = kLeft ? -D : D;  // row of step j: r0 + j * dr
+    uint8_t* orow = (kLeft ? rl : lr) + ro;
+    // chunk c: steps [c*C, c*C + n), pixels [chunk_x, chunk_x + n) in memory order (n <= 0: none)
+    auto chunk_n = [&](int c) { return min(C, len - c * C); };
+    auto chunk_x = [&](int c) { return kLeft ? W - (c * C + chunk_n(c)) : P.x0 + c * C; };
+    auto issue = [&](int c) {  // lane 0
+      const int b = c % NB, n = chunk_n(c);
+      mbar_expect_tx(&bars[w][b], (uint32_t)n * D);
+      bulk_to_smem(cbuf[w][b] + (kLeft ? (C - n) * D : 0), crow + (size_t)chunk_x(c) * D, (uint32_t)n * D, &bars[w][b]);
+    };
+    auto base_of = [&](int c) {  // this lane's step of chunk c
+      if (lane >= chunk_n(c)) return (int)kInvalidShort;
+      return (int)ib[kLeft ? W - 1 - (c * C + lane) : P.x0 + c * C + lane];
+    };
+    ChunkState st{0, false};
+    // parameters of chunk c to every lane (lane j: step j); whether it takes the fast path
+    auto params = [&](int c, int bse) {
+      uint32_t flags, p2;
+      chunk_params(bse, c * C, chunk_n(c), true, P, p2tab, st, flags, p2);
+      const bool fast =
+          __all_sync(kFull, (flags & (kStepValid | kPrevInvalid)) == kStepValid || (c == 0 && lane == 0));
+      par[w][c & 1][lane] = make_uint2(fast ? (uint32_t)(int)(int8_t)(flags & 0xFFu) : flags, p2);
+      return fast;
+    };
+    if (lane == 0) {
+      issue(0);
+      if (nch > 1) issue(1);
+    }
+    bool fast = params(0, base_of(0));
+    int bnext = base_of(1);
+    uint32_t phase = 0u;  // bit b: parity of buffer b's next phase
+    uint32_t L = 0;
+    for (int c = 0; c < nch; ++c) {
+      const int b = c % NB, n = chunk_n(c);
+      if (!mbar_wait_warp(&bars[w][b], (phase >> b) & 1u)) {
+        scan_give_up_mask(bars[w], phase, (1u << b) | (c + 1 < nch ? 1u << ((c + 1) % NB) : 0u));
+        return;
+      }
+      phase ^= 1u << b;
+      __syncwarp();
+      const uint8_t* cb = cbuf[w][b] + lane + r0;
+      const uint2* pq = par[w][c & 1];
+      uint8_t* op = orow + (size_t)chunk_x(c) * D + lane + (kLeft ? (n - 1) * D : 0);  // step 0's byte
+      const int bn = bnext;
+      bnext = base_of(c + 2);  // a chunk ahead (no load past the scanline)
+      const bool run_fast = fast;
+      // groups of R steps; a group's costs and parameters are read during the group before
+      uint32_t cv[R];
+      uint2 q[R];
+      auto read = [&](int g) {
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          cv[j] = cb[(g + j) * dr];
+          q[j] = pq[g + j];
+        }
+      };
+      auto free_buffer = [&]() {
+        fence_proxy_async();  // this lane's reads of the buffer before the copy that refills it
+        __syncwarp();
+        if (lane == 0 && c + 2 < nch) issue(c + 2);
+      };
+      read(0);
+      fast = params(c + 1, bn);
+      if (run_fast) {  // a full chunk (a short one has skipped steps)
+#pragma unroll
+        for (int g = 0; g < C; g += R) {
+          uint32_t cc[R];
+          uint2 qq[R];
+#pragma unroll
+          for (int j = 0; j < R; ++j) {
+            cc[j] = cv[j];
+            qq[j] = q[j];
+          }
+          if (g + R < C) read(g + R);
+          if (g + R == C) free_buffer();
+#pragma unroll
+          for (int j = 0; j < R; ++j) {
+            uint32_t Ls = L;
+            scan_step_fast(Ls, cc[j], (int)qq[j].x, qq[j].y, P.p1);
+            L = (g + j == 0 && c == 0) ? cc[0] : Ls;  // the first pixel of the scanline starts it
+            op[(g + j) * dr] = (uint8_t)L;
+          }
+        }
+      } else {
+        for (int g = 0; g < C; g += R) {
+          if (g) read(g);
+#pragma unroll
+          for (int j = 0; j < R; ++j) {
+            uint32_t Ls = L;
+            scan_step(Ls, cv[j], q[j].x, q[j].y, P.p1);
+            L = (g + j == 0 && c == 0) ? cv[0] : Ls;
+            // a skipped step past a short chunk keeps L: it rewrites the chunk's last pixel
+            op[min(g + j, n - 1) * dr] = (uint8_t)L;
+          }
+        }
+        free_buffer();
+      }
+    }
   };
-  auto base_of = [&](int c) {  // this lane's step of chunk c
-    const int n = chunk_n(c);
-    if (lane >= n) return (int)kInvalidShort;
-    const int x = dir == 0 ? P.x0 + c * C + lane : W - 1 - (c * C + lane);
-    return (int)ib[x];
-  };
-  ChunkState st{0, false};
-  // packed step parameters of chunk c (lane j: step j) and whether it takes the fast path
-  auto params = [&](int c, int bse, uint32_t& pk, bool& fast) {
-    uint32_t flags, p2;
-    chunk_params(bse, c * C, chunk_n(c), true, P, p2tab, st, flags, p2);
-    pk = (p2 << 10) | flags;
-    fast = __all_sync(kFull, (flags & (kStepValid | kPrevInvalid)) == kStepValid || (c == 0 && lane == 0));
-  };
-  if (lane == 0) {
-    issue(0);
-    if (nch > 1) issue(1);
+  if (grp & 1) scan(std::true_type{});
+  else scan(std::false_type{});
+}
+
+// The 32 steps of a column chunk: a step's path costs overwrite its costs at at(j). Groups of kGroup4
+// steps; a group's costs and parameters are read during the group before.
+template <typename At>
+__device__ __forceinline__ void scan_chunk_cols(uint32_t& L, const uint2* par, At at, bool fast, bool first,
+                                                uint32_t p1) {
+  constexpr int C = kScanChunk, R = kGroup4;
+  uint32_t cv[R];
+  uint2 q[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    cv[j] = *at(j);
+    q[j] = par[j];
   }
-  uint32_t pk;
-  bool fast;
-  params(0, base_of(0), pk, fast);
-  int bnext = base_of(1);
-  uint32_t phase = 0u;  // bit b: parity of buffer b's next phase
-  uint32_t L = 0;
-  for (int c = 0; c < nch; ++c) {
-    const int b = c % NB, n = chunk_n(c);
-    if (!mbar_wait_warp(&bars[w][b], (phase >> b) & 1u)) {
-      scan_give_up_mask(bars[w], phase, (1u << b) | (c + 1 < nch ? 1u << ((c + 1) % NB) : 0u));
-      return;
-    }
-    phase ^= 1u << b;
-    __syncwarp();
-    const uint8_t* cb = cbuf[w][b] + lane;
-    const int r0 = dir == 0 ? 0 : (C - 1) * D, dr = dir == 0 ? D : -D;  // row of step j: r0 + j * dr
-    uint32_t cvr[C];
+  auto chunk = [&](auto step) {
 #pragma unroll
-    for (int j = 0; j < C; ++j) cvr[j] = cb[r0 + j * dr];
-    fence_proxy_async();  // this lane's reads of the buffer before the copy that refills it
-    __syncwarp();
-    if (lane == 0 && c + 2 < nch) issue(c + 2);
-    uint8_t* op = orow + (size_t)chunk_x(c) * D + lane + (dir == 0 ? 0 : (n - 1) * D);  // step 0's byte
-    const int od = dir == 0 ? D : -D;
-    const int bn = bnext;
-    bnext = base_of(c + 2);  // a chunk ahead (no load past the scanline)
-    // this chunk's step parameters to every lane
-    par[w][lane] = pk;
-    __syncwarp();
-    uint32_t q[C];
+    for (int g = 0; g < C; g += R) {
+      uint32_t cc[R];
+      uint2 qq[R];
 #pragma unroll
-    for (int j = 0; j < C; ++j) q[j] = par[w][j];
-    __syncwarp();
-    if (fast) {  // a full chunk (a short one has skipped steps)
-      params(c + 1, bn, pk, fast);
-#pragma unroll
-      for (int j = 0; j < C; ++j) {
-        uint32_t Ls = L;
-        scan_step_fast(Ls, cvr[j], (int)(int8_t)(q[j] & 0xFFu), q[j] >> 10, P.p1);
-        L = (j == 0 && c == 0) ? cvr[0] : Ls;  // the first pixel of the scanline starts it
-        op[j * od] = (uint8_t)L;
+      for (int j = 0; j < R; ++j) {
+        cc[j] = cv[j];
+        qq[j] = q[j];
       }
-    } else {
-      params(c + 1, bn, pk, fast);
+      if (g + R < C) {
 #pragma unroll
-      for (int j = 0; j < C; ++j) {
-        uint32_t Ls = L;
-        scan_step(Ls, cvr[j], q[j] & 0x3FFu, q[j] >> 10, P.p1);
-        L = (j == 0 && c == 0) ? cvr[0] : Ls;
-        // a skipped step past a short chunk keeps L: it rewrites the chunk's last pixel
-        op[min(j, n - 1) * od] = (uint8_t)L;
+        for (int j = 0; j < R; ++j) {
+          cv[j] = *at(g + R + j);
+          q[j] = par[g + R + j];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        step(g + j, cc[j], qq[j]);
+        *at(g + j) = (uint8_t)L;
       }
     }
+  };
+  if (fast) {
+    chunk([&](int, uint32_t c, uint2 q) { scan_step_fast(L, c, (int)q.x, q.y, p1); });
+  } else {
+    chunk([&](int j, uint32_t c, uint2 q) {
+      if (j == 0 && first) L = c;
+      else scan_step(L, c, q.x, q.y, p1);
+    });
   }
 }
 
@@ -237,11 +311,12 @@ __global__ void __launch_bounds__(32 * WPB) k_hscan_init4(const uint8_t* __restr
 // tensor-map boxes of 32 rows x 32 bytes, as in k_vscan_plain4: PASS 1 boxes end at rows H - 32c
 // (the last one starts above row 0 and reads zeros there; its steps past row 0 are marked
 // skipped), PASS 3 boxes start at rows 32c. A step's path costs overwrite its costs in the box,
-// which then leaves with one tensor store (a box that reaches past the column, row by row).
+// which then leaves with one tensor store (a box that reaches past the column, row by row). Chunks
+// of valid bases run scan_step_fast, as in the row scans.
 // ---------------------------------------------------------------------------------------------
 // m_out / out: the volume the pass stores (bt or tb) as a tensor map and as a pointer.
 template <int WPB, int PASS>
-__global__ void __launch_bounds__(32 * WPB)
+__global__ void __launch_bounds__(32 * WPB, 1)
     k_vscan_init4(const __grid_constant__ CUtensorMap m_cost, const __grid_constant__ CUtensorMap m_out,
                   const int16_t* __restrict__ init_l, const int16_t* __restrict__ init_r, uint8_t* __restrict__ out,
                   InitParams P) {
@@ -251,7 +326,7 @@ __global__ void __launch_bounds__(32 * WPB)
   constexpr bool kUp = PASS == 1;
   __shared__ __align__(1024) uint8_t cbuf[WPB][NB][BOX];
   __shared__ __align__(8) uint64_t bars[WPB][NB];
-  __shared__ __align__(16) uint32_t par[WPB][2][C];
+  __shared__ __align__(16) uint2 par[WPB][C];
   __shared__ uint32_t p2tab[kP2Tab];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) {
@@ -298,8 +373,8 @@ __global__ void __launch_bounds__(32 * WPB)
     if (c + 1 < nch) bnext = base_of(c + 1);
     uint32_t flags, p2;
     chunk_params(bcur, c * C, n, false, P, p2tab, st, flags, p2);
-    par[w][0][lane] = flags;
-    par[w][1][lane] = p2;
+    const bool fast = __all_sync(kFull, (flags & (kStepValid | kPrevInvalid)) == kStepValid);
+    par[w][lane] = make_uint2(fast ? (uint32_t)(int)(int8_t)(flags & 0xFFu) : flags, p2);
     if (!mbar_wait_warp(&bars[w][b], (phase >> b) & 1u)) {
       scan_give_up_mask(bars[w], phase, (1u << b) | (c + 1 < nch ? 1u << ((c + 1) % NB) : 0u));
       if (lane == 0) bulk_wait_all();
@@ -313,22 +388,8 @@ __global__ void __launch_bounds__(32 * WPB)
       const int r = kUp ? C - 1 - j : j;
       return box + r * D + (box_sw<D>(r) ? lo1 : lo0);
     };
-    // the chunk's step parameters and this lane's costs in registers: the chain below touches no
-    // memory but the stores of its results
-    uint32_t fl[C], pp[C], cvr[C];
-#pragma unroll
-    for (int j = 0; j < C; ++j) {
-      fl[j] = par[w][0][j];
-      pp[j] = par[w][1][j];
-      cvr[j] = *at(j);
-    }
     // all 32 steps run (steps past a short last chunk are marked skipped)
-#pragma unroll
-    for (int j = 0; j < C; ++j) {
-      if (c == 0 && j == 0) L = cvr[0];
-      else scan_step(L, cvr[j], fl[j], pp[j], P.p1);
-      *at(j) = (uint8_t)L;
-    }
+    scan_chunk_cols(L, par[w], at, fast, c == 0, P.p1);
     fence_proxy_async();
     __syncwarp();
     const int y0 = box_y(c);
@@ -445,9 +506,11 @@ __global__ void __launch_bounds__(128) k_wta_init4(const uint8_t* __restrict__ b
 // Top-to-bottom scan of a 32-disparity level with the WTA: as k_vscan_init4 with PASS 3, but a chunk's
 // pixels take their WTA, one lane each, from the chunk's path costs and the boxes of the three stored
 // paths, so the level needs no top-to-bottom volume and moves 4 bytes a voxel where PASS 3 and
-// k_wta_init4 move 6; it can only follow the row scans, where PASS 3 runs beside them.
+// k_wta_init4 move 6; it can only follow the row scans, where PASS 3 runs beside them. Bound by issue and
+// by the steps' chains: 24 warps an SM (80 registers; 12 at 135, 32 spill) and scan_step_fast took the
+// 4800x3409 pyramid's three launches 1637 -> 1290 us.
 template <int WPB>
-__global__ void __launch_bounds__(32 * WPB)
+__global__ void __launch_bounds__(32 * WPB, 24 / WPB)
     k_vscan_wta_init4(const __grid_constant__ CUtensorMap m_cost, const __grid_constant__ CUtensorMap m_bt,
                       const __grid_constant__ CUtensorMap m_lr, const __grid_constant__ CUtensorMap m_rl,
                       const int16_t* __restrict__ init_l, const int16_t* __restrict__ init_r,
@@ -455,7 +518,7 @@ __global__ void __launch_bounds__(32 * WPB)
   constexpr int D = kLevelRange, C = kScanChunk, BOX = C * D, NB = 3;
   __shared__ __align__(1024) uint8_t cbuf[WPB][NB + 3][BOX];  // cost; bt, lr, rl
   __shared__ __align__(8) uint64_t bars[WPB][NB + 1];         // bars[NB]: the stored paths
-  __shared__ __align__(16) uint32_t par[WPB][2][C];
+  __shared__ __align__(16) uint2 par[WPB][C];
   __shared__ uint32_t p2tab[kP2Tab];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) {
@@ -511,8 +574,8 @@ __global__ void __launch_bounds__(32 * WPB)
     if (c + 1 < nch) bnext = base_of(c + 1);
     uint32_t flags, p2;
     chunk_params(bcur, c * C, min(C, H - c * C), false, P, p2tab, st, flags, p2);
-    par[w][0][lane] = flags;
-    par[w][1][lane] = p2;
+    const bool fast = __all_sync(kFull, (flags & (kStepValid | kPrevInvalid)) == kStepValid);
+    par[w][lane] = make_uint2(fast ? (uint32_t)(int)(int8_t)(flags & 0xFFu) : flags, p2);
     if (!mbar_wait_warp(&bars[w][b], (phase >> b) & 1u)) {
       scan_give_up_mask(bars[w], phase, (1u << NB) | (1u << b) | (c + 1 < nch ? 1u << ((c + 1) % NB) : 0u));
       return;
@@ -521,19 +584,7 @@ __global__ void __launch_bounds__(32 * WPB)
     __syncwarp();
     uint8_t* box = cbuf[w][b];
     auto at = [&](int j) { return box + j * D + (box_sw<D>(j) ? lo1 : lo0); };
-    uint32_t fl[C], pp[C], cvr[C];
-#pragma unroll
-    for (int j = 0; j < C; ++j) {
-      fl[j] = par[w][0][j];
-      pp[j] = par[w][1][j];
-      cvr[j] = *at(j);
-    }
-#pragma unroll
-    for (int j = 0; j < C; ++j) {
-      if (c == 0 && j == 0) L = cvr[0];
-      else scan_step(L, cvr[j], fl[j], pp[j], P.p1);
-      *at(j) = (uint8_t)L;
-    }
+    scan_chunk_cols(L, par[w], at, fast, c == 0, P.p1);
     __syncwarp();  // the chunk's path costs, written by disparity, are read by pixel
     if (!mbar_wait_warp(&bars[w][NB], (phase >> NB) & 1u)) {
       scan_give_up_mask(bars[w], phase, (1u << NB) | (c + 1 < nch ? 1u << ((c + 1) % NB) : 0u));
