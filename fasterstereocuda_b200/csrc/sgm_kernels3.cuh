@@ -34,6 +34,15 @@ __device__ __forceinline__ uint32_t widen_hi(uint32_t v) { return __byte_perm(v,
 // Low bytes of the four halves of (w0, w1) -> one 32-bit word of u8 path costs.
 __device__ __forceinline__ uint32_t narrow(uint32_t w0, uint32_t w1) { return __byte_perm(w0, w1, 0x6420); }
 
+// Sums of the bytes of four words: lo = S(0) | S(2) << 16, hi = S(1) | S(3) << 16. A word is its even
+// bytes + 256 times its odd ones, so the sum of the words modulo 2^32 gives lo once hi is known: four byte
+// permutes less than widening both halves.
+__device__ __forceinline__ void sum4_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t e, uint32_t& lo, uint32_t& hi) {
+  hi = __byte_perm(a, 0u, 0x4341u) + __byte_perm(b, 0u, 0x4341u) + __byte_perm(c, 0u, 0x4341u) +
+       __byte_perm(e, 0u, 0x4341u);
+  lo = a + b + c + e - (hi << 8);
+}
+
 // Raw per-thread slices: NR 32-bit words (4*NR bytes, 4-, 8- or 16*n-byte aligned).
 template <int NR>
 __device__ __forceinline__ void ld_slice(const uint8_t* __restrict__ p, uint32_t (&r)[NR]) {

@@ -99,7 +99,7 @@ __device__ __forceinline__ void scan_step_fast(uint32_t& L, uint32_t c, int s, u
   const uint32_t b = __shfl_sync(kFull, Lp, i2 & 31);
   const uint32_t A = (unsigned)i1 < 32u ? a : kInvalidCost;
   const uint32_t B = (unsigned)i2 < 32u ? b : kInvalidCost;
-  const uint32_t t = __vimin3_u32(min(L, m + p2), A, B);
+  const uint32_t t = __vimin3_u32(__viaddmin_u32(m, p2, L), A, B);
   L = c + t - m;
 }
 
@@ -438,12 +438,7 @@ __device__ __forceinline__ float init_wta_rows(const uint8_t* a, const uint8_t* 
     const uint32_t wa[4] = {va.x, va.y, va.z, va.w}, wb[4] = {vb.x, vb.y, vb.z, vb.w};
     const uint32_t wc[4] = {vc.x, vc.y, vc.z, vc.w}, we[4] = {ve.x, ve.y, ve.z, ve.w};
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      lo[4 * q + t] = __byte_perm(wa[t], 0u, 0x4240u) + __byte_perm(wb[t], 0u, 0x4240u) +
-                      __byte_perm(wc[t], 0u, 0x4240u) + __byte_perm(we[t], 0u, 0x4240u);
-      hi[4 * q + t] = __byte_perm(wa[t], 0u, 0x4341u) + __byte_perm(wb[t], 0u, 0x4341u) +
-                      __byte_perm(wc[t], 0u, 0x4341u) + __byte_perm(we[t], 0u, 0x4341u);
-    }
+    for (int t = 0; t < 4; ++t) sum4_bytes(wa[t], wb[t], wc[t], we[t], lo[4 * q + t], hi[4 * q + t]);
   }
   uint32_t mm = __vminu2(lo[0], hi[0]);
 #pragma unroll
@@ -886,13 +881,11 @@ __device__ __forceinline__ float plain_wta_rows(const uint8_t* a, const uint8_t*
     for (int t = 0; t < 4; ++t) {
       const int d0 = 16 * q + 4 * t;  // the word's first disparity
       // lo = S(d0) | S(d0 + 2) << 16, hi = S(d0 + 1) | S(d0 + 3) << 16
-      const uint32_t lo = __byte_perm(wa[t], 0u, 0x4240u) + __byte_perm(wb[t], 0u, 0x4240u) +
-                          __byte_perm(wc[t], 0u, 0x4240u) + __byte_perm(we[t], 0u, 0x4240u);
-      const uint32_t hi = __byte_perm(wa[t], 0u, 0x4341u) + __byte_perm(wb[t], 0u, 0x4341u) +
-                          __byte_perm(wc[t], 0u, 0x4341u) + __byte_perm(we[t], 0u, 0x4341u);
+      uint32_t lo, hi;
+      sum4_bytes(wa[t], wb[t], wc[t], we[t], lo, hi);
       const uint32_t dlo = (uint32_t)(d0 & 63) | ((uint32_t)((d0 + 2) & 63) << 16);
       const uint32_t dhi = dlo + 0x10001u;
-      const uint32_t klo = (lo << 6) | (dlo ^ flip), khi = (hi << 6) | (dhi ^ flip);
+      const uint32_t klo = lo * 64u + (dlo ^ flip), khi = hi * 64u + (dhi ^ flip);
       if (d0 < SPLIT) acc0 = __vimin3_u16x2(acc0, klo, khi);
       else acc1 = __vimin3_u16x2(acc1, klo, khi);
     }

@@ -133,10 +133,8 @@ __device__ __forceinline__ float wta256(const uint8_t* a, const uint8_t* b, cons
     const uint32_t wc[4] = {vc.x, vc.y, vc.z, vc.w}, we[4] = {ve.x, ve.y, ve.z, ve.w};
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      const uint32_t sl = __byte_perm(wa[t], 0u, 0x4240u) + __byte_perm(wb[t], 0u, 0x4240u) +
-                          __byte_perm(wc[t], 0u, 0x4240u) + __byte_perm(we[t], 0u, 0x4240u);
-      const uint32_t sh = __byte_perm(wa[t], 0u, 0x4341u) + __byte_perm(wb[t], 0u, 0x4341u) +
-                          __byte_perm(wc[t], 0u, 0x4341u) + __byte_perm(we[t], 0u, 0x4341u);
+      uint32_t sl, sh;
+      sum4_bytes(wa[t], wb[t], wc[t], we[t], sl, sh);
       lo[t] = min16x2(lo[t], sl * 64u + kb);
       hi[t] = min16x2(hi[t], sh * 64u + kb);
     }
