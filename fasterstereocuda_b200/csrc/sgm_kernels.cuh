@@ -1435,7 +1435,10 @@ __global__ void __launch_bounds__(256) k_dilation(const T* __restrict__ in, T* _
 
 // ---------------------------------------------------------------------------------------------
 // Small-region removal (reference StereoCudaImpl.cpp:32-125, 463-498) as connected-component
-// labelling: union-find over 4-neighbours within a strip, roots = smallest pixel index.
+// labelling: union-find over 4-neighbours within a strip, roots = smallest pixel index. The nodes
+// are horizontal runs of connected pixels: two runs in touch are joined once, not once per pixel, and
+// a run adds its length to its root, not every pixel a one. Bound by the chains of dependent reads
+// and the atomics of a few roots: 450x375, unions 17.0 -> 12.5 us, sizes 10.6 -> 4.5 us.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ bool peaks_adjacent(float a, float b, int abs_mode) {
   const float d = __fsub_rn(a, b);
@@ -1444,7 +1447,7 @@ __device__ __forceinline__ bool peaks_adjacent(float a, float b, int abs_mode) {
   return (t < 0 ? -t : t) <= 1;
 }
 
-// Root of p. Reads go to L2 (ld.global.cg): parents are rewritten by atomics from other SMs.
+// Root of p. Reads go to L2 (ld.global.cg): parents are rewritten by other SMs.
 __device__ __forceinline__ int cc_find(const int* label, int p) {
   int q = __ldcg(label + p);
   while (q != p) {
@@ -1454,41 +1457,69 @@ __device__ __forceinline__ int cc_find(const int* label, int p) {
   return p;
 }
 
+// cc_find that points every second node on its way to its grandparent (path halving), for the unions:
+// the plain store may undo a concurrent atomicMin on the same node, but both values are the node's
+// ancestors, and the thread of the atomicMin goes on to join the parent that it displaced.
+__device__ __forceinline__ int cc_find_halving(int* label, int p) {
+  int q = __ldcg(label + p);
+  while (q != p) {
+    const int g = __ldcg(label + q);
+    if (g == q) return q;
+    __stcg(label + p, g);
+    p = g;
+    q = __ldcg(label + p);
+  }
+  return p;
+}
+
 // Row pass: label[i] = first pixel of i's horizontal run of connected pixels (its provisional
-// root), -1 for INVALID pixels and rows >= `rows`; zeroes count. One warp per row, 32 pixels per
-// step: run starts by ballot, the run of the previous step carried across.
+// root), -1 for INVALID pixels and rows >= `rows`; count[i] = the run's length at its first pixel,
+// 0 at the others. One warp per row, 32 pixels per step: run starts by ballot, the run of the
+// previous step and its length so far carried across.
 __device__ __forceinline__ void cc_rows_warp(const float* __restrict__ disp, int* __restrict__ label,
                                              int* __restrict__ count, int W, int H, int rows, int abs_mode, int y) {
   const int lane = threadIdx.x & 31;
   const float* drow = disp + (size_t)y * W;
   int* lrow = label + (size_t)y * W;
   int* crow = count + (size_t)y * W;
-  int carry = -1;
-  float prev_v = kInvalidFloat;
-  bool prev_valid = false;
-  for (int x0 = 0; x0 < W; x0 += 32) {
-    const int x = x0 + lane;
-    const bool in = x < W;
-    const float v = in ? drow[x] : kInvalidFloat;
-    const bool valid = in && y < rows && v != kInvalidFloat;
-    float lv = __shfl_up_sync(kFull, v, 1);
-    bool lvalid = __shfl_up_sync(kFull, (int)valid, 1) != 0;
-    if (lane == 0) {
-      lv = prev_v;
-      lvalid = prev_valid;
+  int carry = -1, carry_len = 0;
+  bool carry_valid = false;
+  constexpr int U = 4;  // steps whose pixels are read at once
+  for (int xb = 0; xb < W; xb += 32 * U) {
+    float vs[U], ls[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int x = xb + 32 * u + lane;
+      vs[u] = x < W && y < rows ? drow[x] : kInvalidFloat;
+      ls[u] = x > 0 && x < W && y < rows ? drow[x - 1] : kInvalidFloat;
     }
-    const bool conn = valid && lvalid && peaks_adjacent(v, lv, abs_mode);
-    const unsigned brk = __ballot_sync(kFull, !conn);
-    const unsigned upto = brk & (0xFFFFFFFFu >> (31 - lane));
-    const int start = upto ? x0 + (31 - __clz(upto)) : carry;
-    if (in) {
-      lrow[x] = valid ? y * W + start : -1;
-      crow[x] = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int x0 = xb + 32 * u, x = x0 + lane;
+      if (x0 >= W) break;
+      const float v = vs[u], lv = ls[u];
+      const bool valid = v != kInvalidFloat;
+      const bool conn = valid && lv != kInvalidFloat && peaks_adjacent(v, lv, abs_mode);
+      const unsigned brk = __ballot_sync(kFull, !conn);  // the first pixels of runs, and INVALID ones
+      const unsigned upto = brk & (0xFFFFFFFFu >> (31 - lane));
+      const int start = upto ? x0 + (31 - __clz(upto)) : carry;
+      const unsigned above = brk & (0xFFFFFFFEu << lane);  // run starts behind this pixel
+      if (x < W) {
+        lrow[x] = valid ? y * W + start : -1;
+        // a run that reaches the last lane gets its length when it ends
+        if (conn || above) crow[x] = conn || !valid ? 0 : __ffs(above) - 1 - lane;
+      }
+      if (brk) {
+        if (lane == 0 && carry >= 0) crow[carry] = carry_valid ? carry_len + __ffs(brk) - 1 : 0;
+        carry = x0 + 31 - __clz(brk);
+        carry_len = 1 + __clz(brk);
+      } else {
+        carry_len += 32;
+      }
+      carry_valid = __ballot_sync(kFull, valid) >> 31;
     }
-    carry = __shfl_sync(kFull, start, 31);
-    prev_v = __shfl_sync(kFull, v, 31);
-    prev_valid = __shfl_sync(kFull, (int)valid, 31) != 0;
   }
+  if (lane == 0 && carry >= 0 && carry < W) crow[carry] = carry_valid ? carry_len : 0;
 }
 
 static __global__ void k_cc_rows(const float* __restrict__ disp, int* __restrict__ label, int* __restrict__ count,
@@ -1499,7 +1530,8 @@ static __global__ void k_cc_rows(const float* __restrict__ disp, int* __restrict
 }
 
 // Vertical pass: unions pixel i with the pixel below it (same strip) when both are valid and
-// adjacent; roots are the smallest pixel index (atomicMin hooks the larger root).
+// adjacent, unless their left neighbours are so too and in the same two runs: then the leftmost such
+// pair does it. Roots are the smallest pixel index (atomicMin hooks the larger root).
 __device__ __forceinline__ void cc_vert_px(const float* __restrict__ disp, int* label, int W, int H, int tiles,
                                            int rows, int abs_mode, int i) {
   const int y = i / W;
@@ -1507,10 +1539,16 @@ __device__ __forceinline__ void cc_vert_px(const float* __restrict__ disp, int* 
   const int q = i + W;
   const float v = disp[i], w = disp[q];
   if (v == kInvalidFloat || w == kInvalidFloat || !peaks_adjacent(w, v, abs_mode)) return;
+  if (i > y * W) {
+    const float lv = disp[i - 1], lw = disp[q - 1];
+    if (lv != kInvalidFloat && lw != kInvalidFloat && peaks_adjacent(v, lv, abs_mode) &&
+        peaks_adjacent(w, lw, abs_mode) && peaks_adjacent(lw, lv, abs_mode))
+      return;
+  }
   int a = i, b = q;
   while (true) {
-    a = cc_find(label, a);
-    b = cc_find(label, b);
+    a = cc_find_halving(label, a);
+    b = cc_find_halving(label, b);
     if (a == b) break;
     if (a > b) { const int t = a; a = b; b = t; }
     const int old = atomicMin(&label[b], a);
@@ -1526,19 +1564,25 @@ static __global__ void k_cc_vert(const float* __restrict__ disp, int* label, int
   cc_vert_px(disp, label, W, H, tiles, rows, abs_mode, i);
 }
 
-__device__ __forceinline__ void cc_count_px(int* label, int* __restrict__ count, int i) {
-  if (label[i] < 0) return;
-  const int r = cc_find(label, i);
+// Sizes: the first pixel of a run that is not its region's root adds the run's length to the root's
+// count (which starts as the length of its own run) and then points to the root.
+__device__ __forceinline__ void cc_count_px(int* label, int* count, int i) {
+  const int p = __ldcg(label + i);
+  if (p < 0 || p == i) return;
+  const int len = __ldcg(count + i);  // nothing is added to a count that is not a root's
+  if (len == 0) return;
+  const int r = cc_find(label, p);
   label[i] = r;
-  atomicAdd(&count[r], 1);
+  atomicAdd(&count[r], len);
 }
 
 // every processed strip has exactly `tiles` rows, so the threshold is the same for all of them
 __device__ __forceinline__ void cc_filter_px(float* __restrict__ disp, const int* __restrict__ label,
                                              const int* __restrict__ count, int W, int tiles, float ratio, int i) {
-  if (label[i] < 0) return;
+  const int p = label[i];  // the run's first pixel, or the root if this is one
+  if (p < 0) return;
   const int threshold = (int)__fmul_rn((float)(W * tiles), ratio);
-  if (count[label[i]] < threshold) disp[i] = kInvalidFloat;
+  if (count[label[p]] < threshold) disp[i] = kInvalidFloat;
 }
 
 static __global__ void k_cc_count(int* label, int* __restrict__ count, int n) {
