@@ -1034,11 +1034,8 @@ int launch_init(sgm_engine* e, const Word* csl, const Word* csr, const int16_t* 
   Q3.image_border(e->W, e->H);
   // thread-per-scanline kernels: uint32 arithmetic (exact for any penalties); WTA rules 0 and 4
   const bool v3_ok = e->ext.init_tie_rule == sgm::kTieLowest || e->ext.init_tie_rule == sgm::kTieRefB200;
-  // the warp-per-scanline row kernel packs P2' into 22 bits; larger penalties take the default
-  const bool pack_ok = e->opt.p1 >= 0 && e->opt.p1 < (1 << 22) && e->opt.p2_init < (1 << 22) && e->ext.p2_div0 < (1 << 22);
   const bool lat = e->latency && e->tuning_is_default();
-  const int want_row = lat ? 4 : e->tune_row_kernel, tune_col = lat ? 4 : e->tune_col_kernel;
-  const int tune_row = want_row == 4 && !pack_ok ? 0 : want_row;
+  const int tune_row = lat ? 4 : e->tune_row_kernel, tune_col = lat ? 4 : e->tune_col_kernel;
   const bool rows3 = v3_ok && (tune_row == 0 || tune_row == 3);
   const bool cols3 = v3_ok && (tune_col == 0 || tune_col == 3);
   const bool rows4 = tune_row == 4, cols4 = tune_col == 4;
