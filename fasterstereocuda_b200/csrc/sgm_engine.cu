@@ -173,7 +173,7 @@ void sgm_set_process_error(const char* msg) { set_error(nullptr, "%s", msg); }
 int64_t sgm_float_wait_timeouts();  // float_sgm.cu
 
 // One matching level (the state of one StereoCuda instance).
-constexpr int kModes = 3;  // kernel modes of a matcher, see KernelMode
+constexpr int kModes = 5;  // kernel modes of a matcher, see KernelMode
 
 // Initialised matchers of the process (single-level ones and pyramids, not a pyramid's levels).
 static std::atomic<int> g_live_matchers{0};
@@ -192,6 +192,8 @@ struct sgm_engine {
   cudaStream_t stream = nullptr;
   cudaStream_t side = nullptr;                       // the bottom-to-top column pass beside the row scans
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // around the side stream's work
+  cudaStream_t side2 = nullptr;                      // with side: the views beside each other (views_beside)
+  cudaEvent_t ev_view[4] = {};                       // costs of view 0, up 0 / end of side, costs of view 1, up 1
   std::string err;
   int64_t launches = 0;
   // device buffers
@@ -224,6 +226,7 @@ struct sgm_engine {
   // variant 4 in place of the default (see KernelMode): 1 as set by hand, 2 without the volume that its
   // column kernels of the 32-disparity levels allocate
   int latency = 0;
+  bool alone = false;  // with latency: no other match shares the GPU (see KernelMode and launch_plain)
   int tune_row_lanes = 0;   // variant 3: lanes per scanline (0: default)
   int tune_col_lanes = 0;
   bool bt_stored = true;    // the last match wrote the bottom->top volume to global memory
@@ -236,7 +239,7 @@ struct sgm_engine {
   } tmap_key[5];
   // img[0], img[1] -> out captured as a CUDA graph after a first direct run (matches without
   // initial disparities or a right map); later matches copy in, launch it, copy out. One graph
-  // per kernel mode (0: the matcher's tuning, 1 and 2: the latency kernels of KernelMode).
+  // per kernel mode (0: the matcher's tuning, 1 .. 4: the latency kernels of KernelMode).
   cudaGraphExec_t gexec[kModes] = {};
   int direct_runs[kModes] = {};
   int64_t graph_launches[kModes] = {};
@@ -297,6 +300,12 @@ struct sgm_engine {
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     ev_fork = ev_join = nullptr;
+    if (side2) cudaStreamDestroy(side2);
+    side2 = nullptr;
+    for (auto& ev : ev_view) {
+      if (ev) cudaEventDestroy(ev);
+      ev = nullptr;
+    }
     ready = false;
   }
 };
@@ -412,6 +421,8 @@ int engine_init(sgm_engine* e, int W, int H, int M, int D, const sgm_option_t* o
   SGM_CUDA_TRY(e, cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking));
   SGM_CUDA_TRY(e, cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
   SGM_CUDA_TRY(e, cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming));
+  SGM_CUDA_TRY(e, cudaStreamCreateWithFlags(&e->side2, cudaStreamNonBlocking));
+  for (auto& ev : e->ev_view) SGM_CUDA_TRY(e, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   const size_t N = e->npix();
   const size_t V = e->vol() * e->nviews();  // the right view's volumes only with the LR check
   for (int i = 0; i < 2; ++i) {
@@ -617,10 +628,10 @@ int launch_cols256(sgm_engine* e, const sgm::PlainParams& P, const sgm::WtaParam
                    cudaStream_t s) {
   const dim3 grid((e->W + sgm::kWpb5 - 1) / sgm::kWpb5, nv);
   const CUtensorMap *mc, *mb, *ml, *mr;
-  int st = volume_map(e, 0, e->cost, nv, &mc);
-  if (!st) st = volume_map(e, 1, e->bt, nv, &mb);
-  if (!st) st = volume_map(e, 2, e->lr, nv, &ml);
-  if (!st) st = volume_map(e, 3, e->rl, nv, &mr);
+  int st = volume_map(e, 0, e->cost, e->nviews(), &mc);
+  if (!st) st = volume_map(e, 1, e->bt, e->nviews(), &mb);
+  if (!st) st = volume_map(e, 2, e->lr, e->nviews(), &ml);
+  if (!st) st = volume_map(e, 3, e->rl, e->nviews(), &mr);
   if (st) return st;
   SGM_CUDA_TRY(e, sgm::prefer_max_shared(sgm::k_vscan_plain256<PASS>));
   return SGM_LAUNCH(e, s, PASS == 1 ? "vpaths_bt_plain" : "vpaths_wta_plain",
@@ -635,10 +646,10 @@ int launch_cols4(sgm_engine* e, const sgm::PlainParams& P, const sgm::WtaParams&
     constexpr int wpb = sgm::vscan_plain4_warps<K>();
     const dim3 grid((e->W + wpb - 1) / wpb, nv);
     const CUtensorMap *mc, *mb, *ml, *mr;
-    int st = volume_map(e, 0, e->cost, nv, &mc);
-    if (!st) st = volume_map(e, 1, e->bt, nv, &mb);
-    if (!st) st = volume_map(e, 2, e->lr, nv, &ml);
-    if (!st) st = volume_map(e, 3, e->rl, nv, &mr);
+    int st = volume_map(e, 0, e->cost, e->nviews(), &mc);
+    if (!st) st = volume_map(e, 1, e->bt, e->nviews(), &mb);
+    if (!st) st = volume_map(e, 2, e->lr, e->nviews(), &ml);
+    if (!st) st = volume_map(e, 3, e->rl, e->nviews(), &mr);
     if (st) return st;
     auto go = [&](auto kern) -> int {
       SGM_CUDA_TRY(e, sgm::prefer_max_shared(kern));
@@ -679,6 +690,55 @@ int fork_join(sgm_engine* e, cudaStream_t s, SideWork side_work, MainWork main_w
   return SGM_OK;
 }
 
+// The two views of a level on three streams: view 0's scans start when its costs are there and run
+// beside the cost kernel of view 1 (which waits for the population counts, they for the integer ALU),
+// and the scans and WTA of the views fill each other's tails. Each of cost, rows, up (bottom to top)
+// and down (top to bottom with the WTA) takes (view, stream).
+template <typename Cost, typename Rows, typename Up, typename Down>
+int views_beside(sgm_engine* e, cudaStream_t s, Cost cost, Rows rows, Up up, Down down) {
+  cudaError_t r = cudaSuccess;
+  int st = SGM_OK;
+  auto ok = [&]() { return !st && r == cudaSuccess; };
+  auto wait = [&](cudaStream_t on, int ev) {
+    if (ok()) r = cudaStreamWaitEvent(on, e->ev_view[ev], 0);
+  };
+  auto mark = [&](cudaStream_t on, int ev) {
+    if (ok()) r = cudaEventRecord(e->ev_view[ev], on);
+  };
+  auto run = [&](auto work, int view, cudaStream_t on) {
+    if (ok()) st = work(view, on);
+  };
+  const cudaStream_t a = e->side, b = e->side2;
+  run(cost, 0, s);
+  mark(s, 0);  // costs of view 0
+  if (!ok()) {
+    SGM_CUDA_TRY(e, r);
+    return st;
+  }
+  SGM_CUDA_TRY(e, cudaStreamWaitEvent(a, e->ev_view[0], 0));
+  r = cudaStreamWaitEvent(b, e->ev_view[0], 0);
+  run(up, 0, b);
+  mark(b, 1);
+  run(rows, 0, a);
+  wait(a, 1);
+  run(down, 0, a);
+  run(cost, 1, s);
+  mark(s, 2);  // costs of view 1
+  wait(b, 2);
+  run(up, 1, b);
+  run(rows, 1, s);
+  // join even after an error, so that a capture in progress is not left with a forked stream
+  const cudaStream_t forked[2] = {b, a};
+  for (int k = 0; k < 2; ++k) {
+    cudaError_t j = cudaEventRecord(e->ev_view[k ? 1 : 3], forked[k]);
+    if (j == cudaSuccess) j = cudaStreamWaitEvent(s, e->ev_view[k ? 1 : 3], 0);
+    if (r == cudaSuccess) r = j;
+    if (k == 0) run(down, 1, s);
+  }
+  SGM_CUDA_TRY(e, st ? cudaSuccess : r);
+  return st;
+}
+
 template <int K, typename Word>
 int launch_plain(sgm_engine* e, const Word* csl, const Word* csr, float* wta) {
   sgm::PlainParams P;
@@ -711,7 +771,30 @@ int launch_plain(sgm_engine* e, const Word* csl, const Word* csr, float* wta) {
   Q.dmax_excl = warp_kernel ? 32 * K : 32 * K - 1;
   Q.dstride = e->npix();
   Q.image_border(e->W, e->H);
+  // The views beside each other for a match alone, where one view gives every SM six columns and four
+  // row scans: smaller views leave SMs idle in each launch, and several matches in flight fill each
+  // other's gaps (957x541 D = 128: 306 us a match for 300). One pair, both views together -> beside: 1242x375 D = 64
+  // 222 -> 212 us, 1024x768 D = 128 535 -> 511, D = 256 1043 -> 933, 1920x1080 D = 64 767 -> 717; 640x480
+  // D = 128 would take 257 for 242, 1000x100 D = 256 226 for 213.
+  const bool beside = by_default && e->latency && e->alone && nv == 2 && e->W >= 6 * e->nsm && e->H >= 2 * e->nsm && !g_prof.on;
+  auto of = [&](int view) {
+    sgm::PlainParams Pv = P;
+    Pv.view0 = view;
+    return Pv;
+  };
+  auto cost_of = [&](int view, cudaStream_t on) -> int {
+    auto ck = sgm::k_cost3<K, Word>;
+    SGM_CUDA_TRY(e, sgm::prefer_max_shared(ck));  // the scans' split of the SM's memory, to run beside them
+    return SGM_LAUNCH(e, on, "cost", ck<<<dim3((e->W + 127) / 128, e->H), 128, 0, on>>>(csl, csr, e->cost, of(view)));
+  };
   if (K == 8 && by_default && narrow_ok && narrow4_ok(P)) {
+    if (beside) {
+      e->bt_stored = true;
+      return views_beside(
+          e, e->stream, cost_of, [&](int v, cudaStream_t on) { return launch_rows256(e, of(v), 1, on); },
+          [&](int v, cudaStream_t on) { return launch_cols256<1>(e, of(v), Q, wta, 1, on); },
+          [&](int v, cudaStream_t on) { return launch_cols256<2>(e, of(v), Q, wta, 1, on); });
+    }
     dim3 cg((e->W + 127) / 128, e->H, nv);
     st = SGM_LAUNCH(e, e->stream, "cost", sgm::k_cost3<K, Word><<<cg, 128, 0, e->stream>>>(csl, csr, e->cost, P));
     e->bt_stored = true;
@@ -720,6 +803,13 @@ int launch_plain(sgm_engine* e, const Word* csl, const Word* csr, float* wta) {
           e, e->stream, [&](cudaStream_t ss) { return launch_cols256<1>(e, P, Q, wta, nv, ss); },
           [&](cudaStream_t ms) { return launch_rows256(e, P, nv, ms); });
     return st ? st : launch_cols256<2>(e, P, Q, wta, nv, e->stream);
+  }
+  if (beside && tune_row == 4 && cols_v4) {
+    e->bt_stored = true;
+    return views_beside(
+        e, e->stream, cost_of, [&](int v, cudaStream_t on) { return launch_rows4<K>(e, of(v), 1, on); },
+        [&](int v, cudaStream_t on) { return launch_cols4<K, 1>(e, of(v), Q, wta, 1, on); },
+        [&](int v, cudaStream_t on) { return launch_cols4<K, 2>(e, of(v), Q, wta, 1, on); });
   }
   if (((tune_row == 3 || tune_row == 0) && v3_ok) || tune_row == 4) {
     dim3 cg((e->W + 127) / 128, e->H, nv);
@@ -1394,22 +1484,30 @@ struct HostCall {
   HostCall(const HostCall&) = delete;
   HostCall& operator=(const HostCall&) = delete;
   bool latency() const { return n <= kLatencyInFlight; }
+  bool alone() const { return n == 1; }
   bool (*poll() const)() { return latency() ? few_host_calls : nullptr; }
 };
 
 // Latency kernels (sgm_engine::latency: want, 0 for none) on the given engines for the scope of one
-// match when every engine is at the default tuning; mode() is the graph slot to use.
+// match when every engine is at the default tuning; alone: the match probably has the GPU to itself;
+// mode() is the graph slot to use.
 struct KernelMode {
   sgm_engine* const* lv;
   int n, on = 0;
-  KernelMode(sgm_engine* const* levels, int count, int want) : lv(levels), n(count) {
+  KernelMode(sgm_engine* const* levels, int count, int want, bool alone) : lv(levels), n(count) {
     for (int i = 0; i < n; ++i)
       if (!lv[i]->tuning_is_default()) return;
-    on = want;
-    for (int i = 0; i < n; ++i) lv[i]->latency = on;
+    on = want ? want + (alone ? 2 : 0) : 0;
+    for (int i = 0; i < n; ++i) {
+      lv[i]->latency = want;
+      lv[i]->alone = alone;
+    }
   }
   ~KernelMode() {
-    for (int i = 0; i < n; ++i) lv[i]->latency = 0;
+    for (int i = 0; i < n; ++i) {
+      lv[i]->latency = 0;
+      lv[i]->alone = false;
+    }
   }
   KernelMode(const KernelMode&) = delete;
   KernelMode& operator=(const KernelMode&) = delete;
@@ -1424,6 +1522,7 @@ struct KernelMode {
 // 388 .. 293, 1160 .. 303). With 32 matchers the default kernels lead by 3 to 7 % (D = 64, pyramids), so
 // larger pools keep them. Both give the same bits. Nothing is allocated for it (mode 2).
 bool few_matchers() { return g_live_matchers.load(std::memory_order_relaxed) <= kLatencyInFlight; }
+bool only_matcher() { return g_live_matchers.load(std::memory_order_relaxed) == 1; }
 
 int enqueue_depth(sgm_engine* e, const float* disp, float* depth, const sgm_camera_t& c, cudaStream_t s) {
   const int n = (int)e->npix();
@@ -1697,7 +1796,7 @@ int sgm_match(sgm_handle_t h, const uint8_t* img_left, const uint8_t* img_right,
   const size_t N = h->npix();
   h->launches = 0;
   const HostCall call;
-  const KernelMode km(&h, 1, call.latency() ? 1 : 0);
+  const KernelMode km(&h, 1, call.latency() ? 1 : 0, call.alone());
   // with print_log: per-stage times, printed like the reference's timers (StereoCudaImpl.cpp:
   // 365-460, 530-543); the match then runs its kernels directly instead of as a graph
   h->stage_timing = h->print_log;
@@ -1755,7 +1854,7 @@ int sgm_match_device(sgm_handle_t h, const uint8_t* d_left, const uint8_t* d_rig
     return SGM_ERR_ARG;
   }
   h->launches = 0;
-  const KernelMode km(&h, 1, few_matchers() ? 2 : 0);
+  const KernelMode km(&h, 1, few_matchers() ? 2 : 0, only_matcher());
   if (!d_init_disp_left && !d_disp_right)
     return engine_run(h, d_left, d_right, d_disp_left, (cudaStream_t)stream, km.mode());
   return engine_enqueue(h, d_left, d_right, d_init_disp_left, d_disp_left, d_disp_right, (cudaStream_t)stream);
@@ -1782,7 +1881,7 @@ int sgm_match2(sgm_handle_t h, const uint8_t* img_left, const uint8_t* img_right
   const size_t N = h->npix();
   h->launches = 0;
   const HostCall call;
-  const KernelMode km(&h, 1, call.latency() ? 1 : 0);
+  const KernelMode km(&h, 1, call.latency() ? 1 : 0, call.alone());
   SGM_CUDA_TRY(h, cudaMemcpyAsync(h->img[0], img_left, N, cudaMemcpyHostToDevice, h->stream));
   SGM_CUDA_TRY(h, cudaMemcpyAsync(h->img[1], img_right, N, cudaMemcpyHostToDevice, h->stream));
   if (init_disp_left)
@@ -2034,7 +2133,7 @@ int sgm_pyr_match(sgm_pyr_handle_t h, const uint8_t* img_left, const uint8_t* im
   const size_t N = (size_t)h->W * h->H;
   h->launches = 0;
   const HostCall call;
-  const KernelMode km(h->lv.data(), (int)h->lv.size(), call.latency() ? 1 : 0);
+  const KernelMode km(h->lv.data(), (int)h->lv.size(), call.latency() ? 1 : 0, call.alone());
   if (cudaMemcpyAsync(h->in_l, img_left, N, cudaMemcpyHostToDevice, h->stream) ||
       cudaMemcpyAsync(h->in_r, img_right, N, cudaMemcpyHostToDevice, h->stream))
     return SGM_ERR_CUDA;
@@ -2054,7 +2153,7 @@ int sgm_pyr_match_device(sgm_pyr_handle_t h, const uint8_t* d_left, const uint8_
   if (!h->ready) return SGM_ERR_STATE;
   if (!d_left || !d_right || !d_disp) return SGM_ERR_ARG;
   h->launches = 0;
-  const KernelMode km(h->lv.data(), (int)h->lv.size(), few_matchers() ? 2 : 0);
+  const KernelMode km(h->lv.data(), (int)h->lv.size(), few_matchers() ? 2 : 0, only_matcher());
   return pyr_run(h, d_left, d_right, d_disp, stream ? (cudaStream_t)stream : h->stream, km.mode());
 }
 

@@ -236,6 +236,7 @@ struct PlainParams {
   int x0;      // first column of every scan, max(0, min_d)
   uint32_t p1, p2;
   size_t vstride;  // elements between the views of a volume (H*W*D)
+  int view0 = 0;   // first view of the launch (k_cost3 and the warp-per-scanline scans)
 };
 
 // ---------------------------------------------------------------------------------------------

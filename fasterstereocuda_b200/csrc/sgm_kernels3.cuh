@@ -305,7 +305,7 @@ template <int K, typename Word>
 __global__ void __launch_bounds__(128) k_cost3(const Word* __restrict__ cs_l, const Word* __restrict__ cs_r,
                                                uint8_t* __restrict__ cost, PlainParams P) {
   __shared__ Word win[128 + 32 * K];
-  cost3_block<K, Word>(cs_l, cs_r, cost, P, blockIdx.z, blockIdx.y, blockIdx.x * 128, win);
+  cost3_block<K, Word>(cs_l, cs_r, cost, P, P.view0 + blockIdx.z, blockIdx.y, blockIdx.x * 128, win);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -803,7 +803,7 @@ __global__ void __launch_bounds__(32 * WPB) k_hscan_plain4(const uint8_t* __rest
   const int i = blockIdx.x * WPB + w;
   if (i >= nviews * 2 * H) return;  // the whole warp
   const int grp = i / H, y = i - grp * H;
-  const int view = grp >> 1, dir = grp & 1;
+  const int view = P.view0 + (grp >> 1), dir = grp & 1;
   const int len = W - P.x0;
   if (len <= 0) return;
   const size_t ro = (size_t)view * P.vstride + (size_t)y * W * D;
@@ -939,7 +939,7 @@ __device__ __forceinline__ float plain_wta_rows(const uint8_t* a, const uint8_t*
 template <int K>
 __host__ __device__ constexpr int vscan_plain4_warps() { return K == 4 ? 2 : 4; }
 
-// Vertical scans of a plain level: warp (blockIdx.x * WPB + w) owns column x of view blockIdx.y.
+// Vertical scans of a plain level: warp (blockIdx.x * WPB + w) owns column x of view P.view0 + blockIdx.y.
 // PASS 1: bottom to top over boxes ending at rows H - 32c (the last one starts above row 0 and
 // reads zeros there), storing its path costs (bt) box by box -- the last box row by row. PASS 2:
 // top to bottom over boxes starting at rows 32c, then per box the WTA of its pixels with lane =
@@ -964,7 +964,7 @@ __global__ void __launch_bounds__(32 * vscan_plain4_warps<K>())
   __syncwarp();
   const int W = P.W, H = P.H;
   const int x = blockIdx.x * WPB + w;
-  const int view = blockIdx.y;
+  const int view = P.view0 + blockIdx.y;
   if (x >= W) return;  // the whole warp
   float* dout = disp + (size_t)view * Q.dstride + x;
   if (x < P.x0) {

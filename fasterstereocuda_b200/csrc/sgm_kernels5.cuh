@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(32 * kWpb5) k_hscan_plain256(const uint8_t* __
     mbar_fence_init();
   }
   __syncwarp();
-  const int grp = i / H, y = i - grp * H;
+  const int grp = 2 * P.view0 + i / H, y = i % H;
   const bool rtl = grp & 1;
   const size_t ro = (size_t)(grp >> 1) * P.vstride + (size_t)y * W * D;
   const uint8_t* crow = cost + ro;
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(32 * kWpb5)
   __shared__ __align__(8) uint64_t bars[kWpb5][4];  // 0 .. NB - 1: cost; 3: the stored paths
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int W = P.W, H = P.H, nch = (H + C - 1) / C;
-  const int x = blockIdx.x * kWpb5 + w, view = blockIdx.y;
+  const int x = blockIdx.x * kWpb5 + w, view = P.view0 + blockIdx.y;
   if (x >= W) return;  // the whole warp
   disp += (size_t)view * Q.dstride + x;
   if (x < P.x0) {
