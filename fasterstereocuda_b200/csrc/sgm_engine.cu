@@ -226,6 +226,7 @@ struct sgm_engine {
   // variant 4 in place of the default (see KernelMode): 1 as set by hand, 2 without the volume that its
   // column kernels of the 32-disparity levels allocate
   int latency = 0;
+  bool census_ahead = false;  // the census words are there when ev_view[0] is (see pyr_enqueue)
   bool alone = false;  // with latency: no other match shares the GPU (see KernelMode and launch_plain)
   int tune_row_lanes = 0;   // variant 3: lanes per scanline (0: default)
   int tune_col_lanes = 0;
@@ -1209,6 +1210,28 @@ int launch_init(sgm_engine* e, const Word* csl, const Word* csr, const int16_t* 
                     vk<<<vg, vb, vsmem, e->stream>>>(e->cost, e->lr, e->rl, il, ir, e->bt, wta, P, Q, bt_smem));
 }
 
+// Census words of both images.
+int enqueue_census(sgm_engine* e, const uint8_t* dl_img, const uint8_t* dr_img, cudaStream_t s) {
+  const int W = e->W, H = e->H;
+  // 8 rows per block, or 2 when that leaves fewer blocks than SMs (small pyramid levels)
+  constexpr int RY = sgm::kCensusRows;
+  const bool tall = (long)((W + 511) / 512) * ((H + RY - 1) / RY) * 2 >= e->nsm;
+  auto go = [&](auto kern, int ry, auto* csl, auto* csr) -> int {
+    dim3 g((W + 511) / 512, (H + ry - 1) / ry, 2), b(128);
+    // the scans' split of the SM's memory, to run beside them
+    if (s != e->stream) SGM_CUDA_TRY(e, sgm::prefer_max_shared(kern));
+    return SGM_LAUNCH(e, s, "census", kern<<<g, b, 0, s>>>(dl_img, dr_img, csl, csr, W, H));
+  };
+  if (e->opt.cs_type == 1) {
+    auto* l = (uint64_t*)e->cs[0];
+    auto* r = (uint64_t*)e->cs[1];
+    return tall ? go(sgm::k_census4<uint64_t, 4, 3, RY>, RY, l, r) : go(sgm::k_census4<uint64_t, 4, 3, 2>, 2, l, r);
+  }
+  auto* l = (uint32_t*)e->cs[0];
+  auto* r = (uint32_t*)e->cs[1];
+  return tall ? go(sgm::k_census4<uint32_t, 2, 2, RY>, RY, l, r) : go(sgm::k_census4<uint32_t, 2, 2, 2>, 2, l, r);
+}
+
 // Enqueues one full match of this level on s. Inputs/outputs are dense device arrays.
 // roi_l / roi_r: regions of interest of the views (NULL: the whole view), plain levels only.
 int engine_enqueue(sgm_engine* e, const uint8_t* dl_img, const uint8_t* dr_img, const int16_t* dinit, float* dout,
@@ -1252,24 +1275,8 @@ int engine_enqueue(sgm_engine* e, const uint8_t* dl_img, const uint8_t* dr_img, 
   int st = SGM_OK;
   // census of both images
   stage_mark(e, "census");
-  {
-    // 8 rows per block, or 2 when that leaves fewer blocks than SMs (small pyramid levels)
-    constexpr int RY = sgm::kCensusRows;
-    const bool tall = (long)((W + 511) / 512) * ((H + RY - 1) / RY) * 2 >= e->nsm;
-    auto go = [&](auto kern, int ry, auto* csl, auto* csr) {
-      dim3 g((W + 511) / 512, (H + ry - 1) / ry, 2), b(128);
-      return SGM_LAUNCH(e, e->stream, "census", kern<<<g, b, 0, e->stream>>>(dl_img, dr_img, csl, csr, W, H));
-    };
-    if (e->opt.cs_type == 1) {
-      auto* l = (uint64_t*)e->cs[0];
-      auto* r = (uint64_t*)e->cs[1];
-      st = tall ? go(sgm::k_census4<uint64_t, 4, 3, RY>, RY, l, r) : go(sgm::k_census4<uint64_t, 4, 3, 2>, 2, l, r);
-    } else {
-      auto* l = (uint32_t*)e->cs[0];
-      auto* r = (uint32_t*)e->cs[1];
-      st = tall ? go(sgm::k_census4<uint32_t, 2, 2, RY>, RY, l, r) : go(sgm::k_census4<uint32_t, 2, 2, 2>, 2, l, r);
-    }
-  }
+  if (e->census_ahead) SGM_CUDA_TRY(e, cudaStreamWaitEvent(e->stream, e->ev_view[0], 0));
+  else st = enqueue_census(e, dl_img, dr_img, e->stream);
   // right-view initial disparities when checking consistency at an init level
   const int16_t* dinit_r = nullptr;
   if (!st && dinit && e->opt.do_lr_check) {
@@ -1603,6 +1610,11 @@ namespace {
 int pyr_enqueue(sgm_pyramid* p, const uint8_t* dl, const uint8_t* dr, float* dout, cudaStream_t s) {
   const int L = p->layers;
   int st = SGM_OK;
+  // The census of the next finer level needs only the images: with the latency kernels it runs beside a
+  // level (one 3-level pyramid of 1242x375 through the host API 377 -> 364 us). All of them beside the
+  // coarsest level kept that level waiting (4800x3409: no gain).
+  const bool ahead = p->lv[0]->latency && L > 1 && !g_prof.on;
+  const cudaStream_t q = p->lv[0]->side2;
   for (int n = 1; n < L && !st; ++n) {
     sgm_engine* e = p->lv[n];
     dim3 g((e->W + 127) / 128, e->H);
@@ -1619,6 +1631,19 @@ int pyr_enqueue(sgm_pyramid* p, const uint8_t* dl, const uint8_t* dr, float* dou
     float* o = n == 0 ? dout : p->disp[n];
     const int64_t before = e->launches;
     if (n == 0 && p->depth_mode) o = p->disp0;
+    if (ahead && n > 0) {
+      sgm_engine* f = p->lv[n - 1];
+      if (cudaEventRecord(e->ev_view[1], s) != cudaSuccess || cudaStreamWaitEvent(q, e->ev_view[1], 0) != cudaSuccess)
+        st = SGM_ERR_CUDA;
+      if (!st) st = enqueue_census(f, n == 1 ? dl : p->imgs_l[n - 1], n == 1 ? dr : p->imgs_r[n - 1], q);
+      if (!st && cudaEventRecord(f->ev_view[0], q) != cudaSuccess) st = SGM_ERR_CUDA;
+      if (st) {
+        p->err = f->err;
+        break;
+      }
+      f->census_ahead = true;
+      p->launches++;
+    }
     st = engine_enqueue(e, il, ir, n < L - 1 ? p->init[n] : nullptr, o, nullptr, s);
     if (!st && n == 0 && p->depth_mode) st = enqueue_depth(e, e->depth_src, dout, p->cam0, s);
     p->launches += e->launches - before;
@@ -1636,6 +1661,11 @@ int pyr_enqueue(sgm_pyramid* p, const uint8_t* dl, const uint8_t* dr, float* dou
       if (cudaGetLastError() != cudaSuccess) st = SGM_ERR_CUDA;
     }
   }
+  if (ahead)
+    for (int n = 0; n < L; ++n) p->lv[n]->census_ahead = false;
+  // a failed level leaves the side stream to join, or a capture in progress could not end
+  if (ahead && st && cudaEventRecord(p->lv[0]->ev_view[1], q) == cudaSuccess)
+    cudaStreamWaitEvent(s, p->lv[0]->ev_view[1], 0);
   return st;
 }
 
