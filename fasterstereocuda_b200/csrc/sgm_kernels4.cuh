@@ -117,7 +117,7 @@ __device__ __forceinline__ void scan_step_fast(uint32_t& L, uint32_t c, int s, u
 // how many warps are there to issue them. So the two directions are separate code (constant
 // offsets), the parameters arrive ready to use, and a step's costs and parameters are read from
 // shared memory kGroup4 steps ahead, not a chunk (152 -> 96 registers, 12 -> 20 warps an SM; 80
-// registers spill): 4800x3409 pyramid, three levels of row scans 2432 -> 1990 us beside the
+// registers spill): 4800x3409 pyramid, three levels of row scans 2432 -> 2008 us beside the
 // bottom-to-top columns.
 // ---------------------------------------------------------------------------------------------
 constexpr int kGroup4 = 8;
