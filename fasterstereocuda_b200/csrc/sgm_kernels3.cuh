@@ -102,6 +102,9 @@ struct CopyRing {
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  // Before the ring is left with copies in flight: two copies outstanding to one slot have no defined
+  // order, so the next scanline's must not start beside them.
+  static __device__ __forceinline__ void drain() { asm volatile("cp.async.wait_all;" ::: "memory"); }
   // Waits until all but the newest PF - 1 groups are there and reads `slot`.
   __device__ __forceinline__ void take(int slot, uint32_t (&r)[NR]) const {
     asm volatile("cp.async.wait_group %0;" ::"n"(PF - 1) : "memory");
@@ -1121,6 +1124,7 @@ __device__ __forceinline__ void hpaths3_init_lane(const uint8_t* __restrict__ co
       }
       if (__any_sync(kFull, !narrow_m_ok(m))) s_wide = min(len, s0 + PF);  // 32 bits after this block
     }
+    if (s_wide < len) ring.drain();
   }
   if (s_wide < len) {
     init_go_wide<ND, G>(L, s_wide, P, row, g);
