@@ -58,11 +58,16 @@ class FloatSGM(torch.autograd.Function):
     def forward(ctx, cost, p1, p2, temperature=1.0, grad_enabled=True):
         if not (cost.is_cuda and cost.dtype == torch.float32 and cost.dim() == 4):
             raise ValueError("cost must be a float32 CUDA tensor [B,H,W,D]")
-        cost, p1, p2 = _aligned(cost.contiguous()), p1.contiguous().float(), p2.contiguous().float()
         B, H, W, D = cost.shape
+        dev, n = cost.device, B * H * W
+        # the kernels read, and write the gradients of, one penalty a pixel
+        if p1.numel() != n or p2.numel() != n or p1.device != dev or p2.device != dev:
+            raise ValueError(f"p1 and p2 must be [{B}, {H}, {W}] on {dev} (got {list(p1.shape)} on {p1.device}, "
+                             f"{list(p2.shape)} on {p2.device})")
+        cost, p1, p2 = _aligned(cost.contiguous()), p1.contiguous().float(), p2.contiguous().float()
         lib = _lib()
         vol, rec, scratch = _elems(B, H, W, D)
-        dev, temperature = cost.device, float(temperature)
+        temperature = float(temperature)
         keep = grad_enabled and any(ctx.needs_input_grad)  # else no backward pass: nothing is kept for it
         kept = torch.empty(vol + rec if keep else vol, dtype=torch.float32, device=dev)  # S, then the records
         work = torch.empty(scratch, dtype=torch.float32, device=dev)

@@ -214,3 +214,19 @@ def test_segment_edges_and_disparity_alone(D, H, W):
             assert a.abs().max() == 0, name
             continue
         assert (a.cpu().double() - b).norm() / b.norm() < 1e-3, name
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("shape", [(), (1,), (5, 7), (1, 5, 7), (2, 1, 7), (2, 5, 1), (2, 5, 8), (4, 5, 7), None])
+def test_penalties_of_other_sizes_or_devices_are_refused(shape, grad):
+    """Penalty maps without one value a pixel, or on the host (None): an error before any kernel. On
+    tensors without storage, so that no call can reach a GPU."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from fasterstereocuda_b200.float_sgm import float_sgm
+    with FakeTensorMode():
+        cost = torch.empty(2, 5, 7, 32, device="cuda").requires_grad_(grad)
+        good = torch.empty(2, 5, 7, device="cuda")
+        bad = torch.empty(2, 5, 7) if shape is None else torch.empty(shape, device="cuda")
+        for p1, p2 in ((bad, good), (good, bad)):
+            with pytest.raises(ValueError, match="p1 and p2"):
+                float_sgm(cost, p1, p2)
