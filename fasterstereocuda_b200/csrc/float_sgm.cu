@@ -151,7 +151,8 @@ __device__ __forceinline__ bool locate(const Grid4& q, Line& ln, Geo& g) {
 //   argmin kSeg bytes
 // Slot t of a segment is the t-th pixel in the order in which the adjoint walks it (against the
 // path): position 7 - t on paths of ascending position, t on descending ones.
-// codes: 0 same d, 1 d-1, 2 d+1, 3 jump (the first of equal candidates).
+// codes: 0 same d, 1 d-1, 2 d+1, 3 jump (the first of equal candidates; 0 unless another is smaller, so
+// also where L_q(d) is NaN, after a pixel whose costs are all infinite).
 template <int K>
 using CodeWord = typename std::conditional<K == 2, uint32_t, uint16_t>::type;
 
@@ -219,7 +220,7 @@ __device__ __forceinline__ void fstep_warp(float (&L)[K], const float (&c)[K], f
     t[j] = fminf(fminf(fminf(L[j], lm[j]), lp[j]), jump);
     if constexpr (REC) {
       const int sh = 2 * K * slot + 2 * j;
-      const bool q0 = L[j] != t[j], q1 = q0 && lm[j] != t[j], q2 = q1 && lp[j] != t[j];
+      const bool q0 = t[j] < L[j], q1 = q0 && lm[j] != t[j], q2 = q1 && lp[j] != t[j];
       if (q0) r.code += 1u << sh;
       if (q1) r.code += 1u << sh;
       if (q2) r.code += 1u << sh;

@@ -230,3 +230,103 @@ def test_penalties_of_other_sizes_or_devices_are_refused(shape, grad):
         for p1, p2 in ((bad, good), (good, bad)):
             with pytest.raises(ValueError, match="p1 and p2"):
                 float_sgm(cost, p1, p2)
+
+
+def undefined_aware_adjoint(cost, p1, p2, w):
+    """As first_candidate_adjoint, with the documented handling of values that compare with nothing: a minimum
+    passes over NaN, and a candidate takes the place of "same d" only where it is smaller."""
+    D = cost.shape[-1]
+    pad = torch.nn.functional.pad
+
+    def least(q):
+        m = q[..., :1]
+        for k in range(1, D):
+            m = torch.fmin(m, q[..., k:k + 1])
+        return m
+
+    def chosen(q, m, a, b):
+        t, pick = q, torch.zeros(q.shape, dtype=torch.long)
+        for n, c in enumerate((pad(q, (1, 0), value=np.inf)[..., :-1] + a, pad(q, (0, 1), value=np.inf)[..., 1:] + a,
+                               (m + b).expand_as(q)), 1):
+            pick = torch.where(c < t, n, pick)
+            t = torch.where(c < t, c, t)
+        return pick
+    total = 0
+    states = []
+    for dim, rev in ((1, False), (2, False), (1, True), (2, True)):
+        order = list(range(cost.shape[dim]))[::-1 if rev else 1]
+        L = [cost.select(dim, order[0])]
+        for k in order[1:]:
+            m = least(L[-1])
+            a, b = p1.select(dim, k)[..., None], p2.select(dim, k)[..., None]
+            t = torch.fmin(L[-1], pad(L[-1], (1, 0), value=np.inf)[..., :-1] + a)
+            t = torch.fmin(torch.fmin(t, pad(L[-1], (0, 1), value=np.inf)[..., 1:] + a), m + b)
+            L.append(cost.select(dim, k) + t - m)
+        states.append((dim, order, L))
+        total = total + torch.stack([L[order.index(k)] for k in range(len(order))], dim)
+    weight = torch.softmax(-total, -1)
+    levels = torch.arange(D, dtype=cost.dtype)
+    disp = (weight * levels).sum(-1)
+    g_sum = -w[..., None] * weight * (levels - disp[..., None])
+    gc, g1, g2 = torch.zeros_like(cost), torch.zeros_like(p1), torch.zeros_like(p2)
+    for dim, order, L in states:
+        g = torch.zeros_like(L[0])
+        for i in range(len(order) - 1, -1, -1):
+            k = order[i]
+            g = g + g_sum.select(dim, k)
+            gc.select(dim, k).add_(g)
+            if i == 0:
+                break
+            q = L[i - 1]
+            m = least(q)
+            pick = chosen(q, m, p1.select(dim, k)[..., None], p2.select(dim, k)[..., None])
+            same, dn, up, jump = (torch.where(pick == n, g, 0.0) for n in range(4))
+            g1.select(dim, k).add_((dn + up).sum(-1))
+            g2.select(dim, k).add_(jump.sum(-1))
+            at = (q == m) & ((q == m).cumsum(-1) == 1)  # the lowest k, or none
+            back = same + pad(dn, (0, 1))[..., 1:] + pad(up, (1, 0))[..., :-1]
+            g = torch.where(at, back - (same + dn + up).sum(-1, keepdim=True), back)
+    return disp, gc, g1, g2
+
+
+def masked_inputs(case, D):
+    gen = torch.Generator().manual_seed(D)
+    c = torch.rand(2, 21, 37, D, generator=gen, dtype=torch.float64) * 60
+    if case == "voxels":
+        c[torch.rand(c.shape, generator=gen) < 0.3] = np.inf
+        c[..., 5] = 7.0  # a candidate left in every pixel
+    elif case == "pixel":
+        c[0, 10, 20] = np.inf
+    else:
+        c[0, 10, 20, 3] = np.nan
+    p1 = 10.0 + torch.rand(2, 21, 37, generator=gen, dtype=torch.float64)
+    p2 = 150.0 + torch.rand(2, 21, 37, generator=gen, dtype=torch.float64)
+    w = torch.randn(2, 21, 37, generator=gen, dtype=torch.float64)
+    return [t.float().double() for t in (c, p1, p2, w)]
+
+
+@pytest.mark.parametrize("D", [32, 64])
+def test_masked_cost_model_agrees_with_the_plain_adjoint_where_all_is_finite(D):
+    c, p1, p2, w = masked_inputs("voxels", D)
+    for a, b in zip(undefined_aware_adjoint(c, p1, p2, w), first_candidate_adjoint(c, p1, p2, w)):
+        assert torch.allclose(a, b, rtol=1e-12, atol=1e-12)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("case", ["voxels", "pixel", "nan"])
+def test_masked_costs(case, D):
+    """Infinite costs in some voxels, in all of one pixel, and one NaN: the same undefined entries as the
+    model of the documented order, the others within 1e-3 of it in norm (as the tests above)."""
+    from fasterstereocuda_b200.float_sgm import float_sgm
+    c64, p1, p2, w = masked_inputs(case, D)
+    c, q1, q2 = (t.float().cuda().requires_grad_() for t in (c64, p1, p2))
+    d = float_sgm(c, q1, q2)
+    grads = torch.autograd.grad(d, (c, q1, q2), w.float().cuda())
+    with torch.no_grad():
+        assert torch.equal(torch.nan_to_num(float_sgm(c, q1, q2), nan=-1.0), torch.nan_to_num(d, nan=-1.0))
+    for a, b, name in zip((d.detach(), *grads), undefined_aware_adjoint(c64, p1, p2, w), ("disp", "cost", "p1", "p2")):
+        a = a.cpu().double()
+        assert torch.equal(a.isnan(), b.isnan()), (name, int(a.isnan().sum()), int(b.isnan().sum()))
+        ok = ~b.isnan()
+        assert (a[ok] - b[ok]).norm() <= 1e-3 * b[ok].norm() + 1e-30, name
