@@ -583,6 +583,12 @@ bool narrow4_ok(const sgm::PlainParams& P) {
   return P.p1 <= sgm::kInvalidCost && P.p1 <= P.p2 && P.p2 <= sgm::kMaxPenalty16;
 }
 
+// Sizes of a plain level that take the warp-per-scanline kernels unasked: the cost kernel's rows are its
+// grid's y, and a column starts at byte x * D of a tensor map's row, a 32-bit coordinate. Images past
+// either keep the general kernels.
+bool row_bytes_ok(const sgm_engine* e) { return (size_t)e->W * e->D <= (size_t)INT32_MAX; }
+bool scans4_fit(const sgm_engine* e) { return e->H <= 65535 && row_bytes_ok(e); }
+
 // Warp-per-scanline kernels (variant 4, D <= 128): the row scans, and the column passes (pass 1
 // bottom-to-top, pass 2 top-to-bottom + sum + WTA).
 template <int K>
@@ -755,9 +761,10 @@ int launch_plain(sgm_engine* e, const Word* csl, const Word* csr, float* wta) {
   int st;
   // warp-per-scanline kernels: D <= 128 and the tie rules of their serial WTA; otherwise the
   // default takes their place
-  const bool v4_ok = K <= 4 && (e->ext.tie_rule == sgm::kTieLowest || e->ext.tie_rule == sgm::kTieHighest ||
-                                e->ext.tie_rule == sgm::kTieRefB200);
-  const bool by_default = e->tuning_is_default();
+  const bool v4_ok = K <= 4 && row_bytes_ok(e) &&
+                     (e->ext.tie_rule == sgm::kTieLowest || e->ext.tie_rule == sgm::kTieHighest ||
+                      e->ext.tie_rule == sgm::kTieRefB200);
+  const bool by_default = e->tuning_is_default() && scans4_fit(e);
   const int want_row = by_default && e->latency ? 4 : e->tune_row_kernel;
   const int want_col = by_default && e->latency ? 4 : e->tune_col_kernel;
   const int tune_row = want_row == 4 && !v4_ok ? 0 : want_row;
