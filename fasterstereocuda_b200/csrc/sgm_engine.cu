@@ -1275,8 +1275,12 @@ int engine_enqueue(sgm_engine* e, const uint8_t* dl_img, const uint8_t* dr_img, 
     set_error(&e->err, "initial disparities need using_constant_p2 (the reference launches no aggregation otherwise)");
     return SGM_ERR_UNSUPPORTED;
   }
-  cudaStream_t saved = e->stream;
-  e->stream = s ? s : e->stream;
+  struct OnStream {  // the match's stream for the scope of this call, whichever way it ends
+    sgm_engine* e;
+    cudaStream_t own;
+    ~OnStream() { e->stream = own; }
+  } const on{e, e->stream};
+  if (s) e->stream = s;
   const int W = e->W, H = e->H;
   const size_t N = e->npix();
   int st = SGM_OK;
@@ -1423,7 +1427,6 @@ int engine_enqueue(sgm_engine* e, const uint8_t* dl_img, const uint8_t* dr_img, 
   }
   stage_mark(e, nullptr);
   e->depth_src = (!peaks && ((pf != 0) != (morph != 0))) ? agg : dout;
-  e->stream = saved;
   return st;
 }
 

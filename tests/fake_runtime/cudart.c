@@ -45,7 +45,7 @@ API void fake_fail(const char* name, int after) {
 static cudaError_t done(const char* name) {
   if (fail_after >= 0 && !strcmp(name, fail_name) && fail_after-- == 0) {
     note("FAILED %s", name);
-    return last_error = cudaErrorInvalidResourceHandle;
+    return cudaErrorInvalidResourceHandle;
   }
   return cudaSuccess;
 }
@@ -90,7 +90,9 @@ static cudaError_t launch(const void* f, dim3 g, dim3 b, size_t smem, cudaStream
     return last_error = cudaErrorInvalidConfiguration;
   }
   note("launch %s grid %u %u %u stream %p%s", name_of(f), g.x, g.y, g.z, (void*)s, more);
-  return done("cudaLaunchKernel");
+  const cudaError_t e = done("cudaLaunchKernel");
+  if (e) last_error = e;  /* the one a launch is checked by; other calls' errors are their results */
+  return e;
 }
 API cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void** args, size_t smem, cudaStream_t s) {
   (void)args;
