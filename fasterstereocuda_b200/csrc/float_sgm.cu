@@ -818,9 +818,8 @@ int forward_impl(const float* cost, const float* p1, const float* p2, int B, int
 }
 
 template <int G>
-int backward_impl(const float* cost, const float* p1, const float* p2, int B, int H, int W, float inv_t,
-                  const float* sum, const float* ckpt, const float* grad_disp, float* grad_sum, float* work,
-                  float* grad_cost, float* grad_p1, float* grad_p2, cudaStream_t s) {
+int backward_impl(int B, int H, int W, float inv_t, const float* sum, const float* ckpt, const float* grad_disp,
+                  float* grad_sum, float* work, float* grad_cost, float* grad_p1, float* grad_p2, cudaStream_t s) {
   constexpr int D = G * kBwdK;
   const size_t V = (size_t)B * H * W * D, npix = (size_t)B * H * W;
   constexpr int GS = D / kK;  // lanes per pixel of the soft-argmin kernels
@@ -918,10 +917,10 @@ int sgm_float_backward(const float* cost, const float* p1, const float* p2, int3
     return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const float inv_t = 1.0f / temperature;
-  return D == 64 ? backward_impl<64 / kBwdK>(cost, p1, p2, B, H, W, inv_t, sum, ckpt, grad_disp, grad_sum, work,
-                                             grad_cost, grad_p1, grad_p2, s)
-                 : backward_impl<32 / kBwdK>(cost, p1, p2, B, H, W, inv_t, sum, ckpt, grad_disp, grad_sum, work,
-                                             grad_cost, grad_p1, grad_p2, s);
+  return D == 64 ? backward_impl<64 / kBwdK>(B, H, W, inv_t, sum, ckpt, grad_disp, grad_sum, work, grad_cost, grad_p1,
+                                             grad_p2, s)
+                 : backward_impl<32 / kBwdK>(B, H, W, inv_t, sum, ckpt, grad_disp, grad_sum, work, grad_cost, grad_p1,
+                                             grad_p2, s);
 }
 
 }  // extern "C"

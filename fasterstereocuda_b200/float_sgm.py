@@ -79,24 +79,25 @@ class FloatSGM(torch.autograd.Function):
             return disp
         _check(lib, lib.sgm_float_forward(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D, temperature,
                                           sum_, sum_ + 4 * vol, work.data_ptr(), disp.data_ptr(), stream), "forward")
-        ctx.save_for_backward(cost, p1, p2, kept)
-        ctx.temperature = temperature
+        ctx.save_for_backward(kept)
+        ctx.shapes, ctx.temperature = (cost.shape, p1.shape, p2.shape), temperature
         return disp
 
     @staticmethod
     def backward(ctx, grad_disp):
-        cost, p1, p2, kept = ctx.saved_tensors
-        B, H, W, D = cost.shape
+        (kept,) = ctx.saved_tensors  # S and the records: the inputs are not needed again
+        B, H, W, D = ctx.shapes[0]
         lib = _lib()
         vol, _, scratch = _elems(B, H, W, D)
         g = grad_disp.contiguous().float()
-        work = torch.empty(vol + scratch, dtype=torch.float32, device=cost.device)  # gradient of S, workspace
-        gcost, gp1, gp2 = torch.empty_like(cost), torch.empty_like(p1), torch.empty_like(p2)
+        work = kept.new_empty(vol + scratch)  # gradient of S, workspace
+        gcost, gp1, gp2 = (kept.new_empty(shape) for shape in ctx.shapes)
         sum_, gsum = kept.data_ptr(), work.data_ptr()
-        _check(lib, lib.sgm_float_backward(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D, ctx.temperature,
-                                           sum_, sum_ + 4 * vol, g.data_ptr(), gsum, gsum + 4 * vol,
-                                           gcost.data_ptr(), gp1.data_ptr(), gp2.data_ptr(),
-                                           torch.cuda.current_stream(cost.device).cuda_stream), "backward")
+        # S in the place of the inputs, which the call asks for and does not read
+        _check(lib, lib.sgm_float_backward(sum_, sum_, sum_, B, H, W, D, ctx.temperature, sum_, sum_ + 4 * vol,
+                                           g.data_ptr(), gsum, gsum + 4 * vol, gcost.data_ptr(), gp1.data_ptr(),
+                                           gp2.data_ptr(), torch.cuda.current_stream(kept.device).cuda_stream),
+               "backward")
         return gcost, gp1, gp2, None, None
 
 

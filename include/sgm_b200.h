@@ -305,8 +305,9 @@ SGM_API int sgm_float_disparity(const float* cost, const float* p1, const float*
                                 int32_t D, float temperature, float* sum, float* work, float* disp, void* stream);
 /* No counterpart in the reference. Gradients of sum(grad_disp * disp) with respect to cost, p1
  * and p2 (written, not accumulated); grad_sum [B][H][W][D] and work (sgm_float_workspace_elems
- * floats) are scratch. Each path's gradient is routed by the recorded choices. grad_sum and
- * grad_cost 16-byte aligned. */
+ * floats) are scratch. Each path's gradient is routed by the recorded choices: cost, p1 and
+ * p2 are checked but not read, and may have changed or be any other aligned device memory. grad_sum
+ * and grad_cost 16-byte aligned. */
 SGM_API int sgm_float_backward(const float* cost, const float* p1, const float* p2, int32_t B, int32_t H, int32_t W,
                                int32_t D, float temperature, const float* sum, const float* ckpt,
                                const float* grad_disp, float* grad_sum, float* work, float* grad_cost,

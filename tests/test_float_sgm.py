@@ -330,3 +330,24 @@ def test_masked_costs(case, D):
         assert torch.equal(a.isnan(), b.isnan()), (name, int(a.isnan().sum()), int(b.isnan().sum()))
         ok = ~b.isnan()
         assert (a[ok] - b[ok]).norm() <= 1e-3 * b[ok].norm() + 1e-30, name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64])
+def test_backward_after_the_inputs_changed(D):
+    """The gradients come from what the forward pass recorded: inputs that are overwritten in place
+    before the backward pass neither raise nor change them."""
+    from fasterstereocuda_b200.float_sgm import float_sgm
+    c64, p1, p2, w = masked_inputs("voxels", D)
+    w = w.float().cuda()
+
+    def run(change):
+        leaves = [t.float().cuda().requires_grad_() for t in (c64, p1, p2)]
+        inputs = [t * 1 for t in leaves]
+        d = float_sgm(*inputs)
+        if change:
+            for t in inputs:
+                t.zero_()
+        return torch.autograd.grad(d, leaves, w)
+    for a, b in zip(run(True), run(False)):
+        assert torch.equal(a, b)
