@@ -791,9 +791,9 @@ int launch_plain(sgm_engine* e, const Word* csl, const Word* csr, float* wta) {
     return Pv;
   };
   auto cost_of = [&](int view, cudaStream_t on) -> int {
-    auto ck = sgm::k_cost3<K, Word>;
-    SGM_CUDA_TRY(e, sgm::prefer_max_shared(ck));  // the scans' split of the SM's memory, to run beside them
-    return SGM_LAUNCH(e, on, "cost", ck<<<dim3((e->W + 127) / 128, e->H), 128, 0, on>>>(csl, csr, e->cost, of(view)));
+    // the scans' split of the SM's memory, to run beside them
+    return SGM_LAUNCH(e, on, "cost", sgm::launch_max_shared(sgm::k_cost3<K, Word>, dim3((e->W + 127) / 128, e->H), 128,
+                                                            on, csl, csr, e->cost, of(view)));
   };
   if (K == 8 && by_default && narrow_ok && narrow4_ok(P)) {
     if (beside) {
@@ -1225,8 +1225,8 @@ int enqueue_census(sgm_engine* e, const uint8_t* dl_img, const uint8_t* dr_img, 
   const bool tall = (long)((W + 511) / 512) * ((H + RY - 1) / RY) * 2 >= e->nsm;
   auto go = [&](auto kern, int ry, auto* csl, auto* csr) -> int {
     dim3 g((W + 511) / 512, (H + ry - 1) / ry, 2), b(128);
-    // the scans' split of the SM's memory, to run beside them
-    if (s != e->stream) SGM_CUDA_TRY(e, sgm::prefer_max_shared(kern));
+    if (s != e->stream)  // beside scans: with their split of the SM's memory
+      return SGM_LAUNCH(e, s, "census", sgm::launch_max_shared(kern, g, b, s, dl_img, dr_img, csl, csr, W, H));
     return SGM_LAUNCH(e, s, "census", kern<<<g, b, 0, s>>>(dl_img, dr_img, csl, csr, W, H));
   };
   if (e->opt.cs_type == 1) {
