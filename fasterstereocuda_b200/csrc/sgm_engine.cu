@@ -266,6 +266,9 @@ struct sgm_engine {
   }
 
   int nviews() const { return opt.do_lr_check ? 2 : 1; }
+  // Two views, of which each gives every SM six columns and four row scans: smaller ones leave SMs idle in
+  // each launch when they run beside each other (see launch_plain).
+  bool views_fill() const { return nviews() == 2 && W >= 6 * nsm && H >= 2 * nsm; }
   size_t npix() const { return (size_t)W * H; }
   size_t vol() const { return (size_t)W * H * D; }
   int census_bytes() const { return opt.cs_type == 1 ? 8 : 4; }
@@ -779,12 +782,11 @@ int launch_plain(sgm_engine* e, const Word* csl, const Word* csr, float* wta) {
   Q.dmax_excl = warp_kernel ? 32 * K : 32 * K - 1;
   Q.dstride = e->npix();
   Q.image_border(e->W, e->H);
-  // The views beside each other for a match alone, where one view gives every SM six columns and four
-  // row scans: smaller views leave SMs idle in each launch, and several matches in flight fill each
-  // other's gaps (957x541 D = 128: 306 us a match for 300). One pair, both views together -> beside: 1242x375 D = 64
+  // The views beside each other for a match alone, where they are large enough: several matches in flight
+  // fill each other's gaps (957x541 D = 128: 306 us a match for 300). One pair, both views together -> beside: 1242x375 D = 64
   // 222 -> 212 us, 1024x768 D = 128 535 -> 511, D = 256 1043 -> 933, 1920x1080 D = 64 767 -> 717; 640x480
   // D = 128 would take 257 for 242, 1000x100 D = 256 226 for 213.
-  const bool beside = by_default && e->latency && e->alone && nv == 2 && e->W >= 6 * e->nsm && e->H >= 2 * e->nsm && !g_prof.on;
+  const bool beside = by_default && e->latency && e->alone && e->views_fill() && !g_prof.on;
   auto of = [&](int view) {
     sgm::PlainParams Pv = P;
     Pv.view0 = view;
@@ -1506,14 +1508,19 @@ struct HostCall {
 };
 
 // Latency kernels (sgm_engine::latency: want, 0 for none) on the given engines for the scope of one
-// match when every engine is at the default tuning; alone: the match probably has the GPU to itself;
-// mode() is the graph slot to use.
+// match when every engine is at the default tuning; alone: the match probably has the GPU to itself,
+// which matters, and takes a graph of its own, only where views run beside each other: elsewhere a
+// second caller or matcher that comes or goes would have the same launches recorded twice (450x375: 316 us in
+// place of 158 for the call that did it). mode() is the graph slot to use.
 struct KernelMode {
   sgm_engine* const* lv;
   int n, on = 0;
   KernelMode(sgm_engine* const* levels, int count, int want, bool alone) : lv(levels), n(count) {
     for (int i = 0; i < n; ++i)
       if (!lv[i]->tuning_is_default()) return;
+    bool split = false;
+    for (int i = 0; i < n; ++i) split = split || lv[i]->views_fill();
+    alone = alone && split;
     on = want ? want + (alone ? 2 : 0) : 0;
     for (int i = 0; i < n; ++i) {
       lv[i]->latency = want;
