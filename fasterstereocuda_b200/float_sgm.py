@@ -61,7 +61,7 @@ class FloatSGM(torch.autograd.Function):
         B, H, W, D = cost.shape
         dev, n = cost.device, B * H * W
         # the kernels read, and write the gradients of, one penalty a pixel
-        if p1.numel() != n or p2.numel() != n or p1.device != dev or p2.device != dev:
+        if not (p1.numel() == n == p2.numel() and p1.device == dev == p2.device):
             raise ValueError(f"p1 and p2 must be [{B}, {H}, {W}] on {dev} (got {list(p1.shape)} on {p1.device}, "
                              f"{list(p2.shape)} on {p2.device})")
         cost, p1, p2 = _aligned(cost.contiguous()), p1.contiguous().float(), p2.contiguous().float()
@@ -69,9 +69,8 @@ class FloatSGM(torch.autograd.Function):
         vol, rec, scratch = _elems(B, H, W, D)
         temperature = float(temperature)
         keep = grad_enabled and any(ctx.needs_input_grad)  # else no backward pass: nothing is kept for it
-        kept = torch.empty(vol + rec if keep else vol, dtype=torch.float32, device=dev)  # S, then the records
-        work = torch.empty(scratch, dtype=torch.float32, device=dev)
-        disp = torch.empty((B, H, W), dtype=torch.float32, device=dev)
+        kept = cost.new_empty(vol + rec if keep else vol)  # S, then the records
+        work, disp = cost.new_empty(scratch), cost.new_empty(B, H, W)
         sum_, stream = kept.data_ptr(), torch.cuda.current_stream(dev).cuda_stream
         if not keep:
             _check(lib, lib.sgm_float_disparity(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D, temperature,
@@ -80,24 +79,26 @@ class FloatSGM(torch.autograd.Function):
         _check(lib, lib.sgm_float_forward(cost.data_ptr(), p1.data_ptr(), p2.data_ptr(), B, H, W, D, temperature,
                                           sum_, sum_ + 4 * vol, work.data_ptr(), disp.data_ptr(), stream), "forward")
         ctx.save_for_backward(kept)
-        ctx.shapes, ctx.temperature = (cost.shape, p1.shape, p2.shape), temperature
+        ctx.sizes, ctx.maps, ctx.temperature = (B, H, W, D), (p1.shape, p2.shape), temperature
         return disp
 
     @staticmethod
     def backward(ctx, grad_disp):
         (kept,) = ctx.saved_tensors  # S and the records: the inputs are not needed again
-        B, H, W, D = ctx.shapes[0]
+        B, H, W, D = ctx.sizes
         lib = _lib()
         vol, _, scratch = _elems(B, H, W, D)
         g = grad_disp.contiguous().float()
         work = kept.new_empty(vol + scratch)  # gradient of S, workspace
-        gcost, gp1, gp2 = (kept.new_empty(shape) for shape in ctx.shapes)
+        gcost, gp1, gp2 = kept.new_empty(B, H, W, D), torch.empty_like(g), torch.empty_like(g)
         sum_, gsum = kept.data_ptr(), work.data_ptr()
         # S in the place of the inputs, which the call asks for and does not read
         _check(lib, lib.sgm_float_backward(sum_, sum_, sum_, B, H, W, D, ctx.temperature, sum_, sum_ + 4 * vol,
                                            g.data_ptr(), gsum, gsum + 4 * vol, gcost.data_ptr(), gp1.data_ptr(),
                                            gp2.data_ptr(), torch.cuda.current_stream(kept.device).cuda_stream),
                "backward")
+        if ctx.maps != (g.shape, g.shape):  # maps of another shape with as many values
+            gp1, gp2 = gp1.view(ctx.maps[0]), gp2.view(ctx.maps[1])
         return gcost, gp1, gp2, None, None
 
 

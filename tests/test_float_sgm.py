@@ -351,3 +351,20 @@ def test_backward_after_the_inputs_changed(D):
         return torch.autograd.grad(d, leaves, w)
     for a, b in zip(run(True), run(False)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+def test_penalty_maps_of_another_shape_with_a_value_a_pixel():
+    """Such maps are taken in the order of their values; their gradients have their shape."""
+    from fasterstereocuda_b200.float_sgm import float_sgm
+    c64, p1, p2, w = masked_inputs("voxels", 32)
+    w = w.float().cuda()
+    grads = []
+    for s1, s2 in (((2, 21, 37), (2, 21, 37)), ((2, 1, 21, 37), (2, 21, 37)), ((2 * 21 * 37,), (2, 21, 37, 1))):
+        c, q1, q2 = c64.float().cuda().requires_grad_(), *(p.float().cuda().view(s).requires_grad_()
+                                                          for p, s in ((p1, s1), (p2, s2)))
+        g = torch.autograd.grad(float_sgm(c, q1, q2), (c, q1, q2), w)
+        assert g[1].shape == s1 and g[2].shape == s2
+        grads.append([t.reshape(-1) for t in g])
+    for other in grads[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(grads[0], other))
