@@ -520,8 +520,10 @@ __device__ __forceinline__ void reduce_segment(float (&v)[2 * kSeg], int gl) {
 // warp barrier. As a ring of registers the loads shared scoreboards with younger loads and with the
 // step's shuffles, and a row step took ~750 cycles.
 // Four disparities per lane: with eight, twice the lines fit a warp, but a step is twice the
-// instructions for one warp to issue, and the row scans take as long as their steps do (one 1242x375
-// image, D = 64, backward pass 581 -> 479 us; four 1294 -> 1274 us, and at D = 32 803 -> 722 us).
+// instructions for one warp to issue, and the row scans take as long as their steps do (both with the
+// copies ahead: one 1242x375 image, D = 64, backward pass 581 -> 479 us; four 1294 -> 1274 us, and at
+// D = 32 803 -> 722 us). From the ring of registers with eight: one 627 -> 481, four 1330 -> 1272, but eight
+// 320x240 images 411 -> 426.
 template <int G>
 __global__ void __launch_bounds__(kWarps * 32, 4) k_float_bwd(const BwdArgs a) {
   constexpr int K = kBwdK, D = G * K, FK = D / 32, PF = kBwdPF;

@@ -140,8 +140,8 @@ inline cudaError_t prefer_max_shared(F* fn) {
 
 // One launch of `fn` with that carveout, for kernels that only sometimes run beside such ones: the
 // function itself, and with it every other launch, keeps the default split. As a function attribute the
-// cost kernel's stayed for all later matches, and 32 matchers of 1242x375, D = 64, took 154.2 instead of
-// 152.8 us a match.
+// cost kernel's stayed for all later matches (32 matchers of 1242x375, D = 64, 152.8 -> 154.2 us a match
+// in one run; runs differ by about as much).
 template <typename... P, typename... A>
 inline cudaError_t launch_max_shared(void (*fn)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
   cudaLaunchAttribute split{};

@@ -218,8 +218,7 @@ struct sgm_engine {
   int tune_rows = 0;        // rows per CTA of the row kernels (0: default)
   int tune_cols = 0;        // columns per CTA of the column kernels (0: default)
   int tune_bt_smem = 0;     // 1: keep bottom->top path costs in shared memory when they fit
-  // 0: the default, else 1
-  // whole-row census, 2 chunked, 3 u16x2 per scanline, 4 one warp per scanline
+  // 0: the default, else 1 whole-row census, 2 chunked, 3 u16x2 per scanline, 4 one warp per scanline
   int tune_row_kernel = 0;
   // 0: the default, else 1 plain loads, 2 prefetch ring, 3 u16x2 per column, 4 one warp per column
   int tune_col_kernel = 0;
@@ -1086,8 +1085,8 @@ int init4_cols(sgm_engine* e, const int16_t* il, const int16_t* ir, const sgm::I
 
 // Top to bottom with the WTA, needing no top-to-bottom volume: for the device API, which allocates
 // nothing. Slower than both column directions beside the row scans and a WTA launch after them (one
-// 3-level pyramid of 1242x375 alone 367 against 331 us, three in flight 207 against 197; 4800x3409
-// 5.75 against 5.32 ms, 4.99 against 4.83): a level stays with those once it holds the volume.
+// 3-level pyramid of 1242x375 alone 349 against 309 us, three in flight 190 against 177; 4800x3409
+// 5.12 against 4.81 ms, 4.41 against 4.39): a level stays with those once it holds the volume.
 inline int init4_cols_wta(sgm_engine* e, const int16_t* il, const int16_t* ir, float* wta, const sgm::InitParams& P,
                           const sgm::WtaParams& Q, cudaStream_t s) {
   const int nv = e->nviews();
@@ -1540,11 +1539,13 @@ struct KernelMode {
 
 // The device API (sgm_match_device, sgm_pyr_match_device) does not wait, so it cannot know how much of
 // its work is in flight. While at most kLatencyInFlight matchers are initialised in the process, no
-// more than that many matches can share the GPU, and the latency kernels are the faster ones at
-// every number of them (us a match with one .. eight matchers in flight on one B200: 450x375, D = 64
-// 110 .. 57, default kernels 414 .. 78; 1242x375, D = 64 220 .. 149, 767 .. 153; 957x541, D = 128
-// 388 .. 293, 1160 .. 303). With 32 matchers the default kernels lead by 3 to 7 % (D = 64, pyramids), so
-// larger pools keep them. Both give the same bits. Nothing is allocated for it (mode 2).
+// more than that many matches can share the GPU, and the latency kernels are the faster ones or level
+// (us a match with one .. eight matchers in flight on one B200, default kernels behind: 320x240, D = 64
+// 68 .. 28, 254 .. 45; 1242x375, D = 64 202 .. 155, 778 .. 155; D = 128 349 .. 279, 1125 .. 301), but for
+// large levels at D <= 64 with four or more in flight, which fill the GPU either way (1920x1080, D = 64
+// eight 679 for 665; 3000x2000 four 1995 for 1943, one 1998 for 3251). With 32 matchers the default
+// kernels lead by 3 to 7 % (D = 64, pyramids), so larger pools keep them, also a pool of which one is
+// used at a time. Both give the same bits. Nothing is allocated for it (mode 2).
 bool few_matchers() { return g_live_matchers.load(std::memory_order_relaxed) <= kLatencyInFlight; }
 bool only_matcher() { return g_live_matchers.load(std::memory_order_relaxed) == 1; }
 

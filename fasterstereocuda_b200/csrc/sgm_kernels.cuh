@@ -1439,7 +1439,7 @@ __global__ void __launch_bounds__(256) k_dilation(const T* __restrict__ in, T* _
 // labelling: union-find over 4-neighbours within a strip, roots = smallest pixel index. The nodes
 // are horizontal runs of connected pixels: two runs in touch are joined once, not once per pixel, and
 // a run adds its length to its root, not every pixel a one. Bound by the chains of dependent reads
-// and the atomics of a few roots: 450x375, unions 17.0 -> 12.5 us, sizes 10.6 -> 4.5 us.
+// and the atomics of a few roots: 450x375, unions 17.0 -> 11.5 us, sizes 10.6 -> 4.6 us.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ bool peaks_adjacent(float a, float b, int abs_mode) {
   const float d = __fsub_rn(a, b);

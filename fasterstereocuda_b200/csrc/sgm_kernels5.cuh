@@ -7,10 +7,11 @@
 // that all 2880 row scans of a 1280x720 pair are resident at once; with sixteen the last 8 % of them
 // ran alone. One 256-byte bulk copy per image row instead of the box was bound by the copies' issue
 // (389 us bottom to top).
-// One pair of 1280x720 alone: rows and bottom-to-top columns side by side 591 us (2.8 GB, 4.8 TB/s),
-// top to bottom with the WTA 343 us (1.9 GB, 5.5 TB/s); the lane-per-disparity kernels they replace
-// took 1582 us for the rows and 1961 us for the columns (32-bit values, plain loads per step). With
-// three pairs in flight a match takes 1.02 ms, 5.1 TB/s of its 5.2 GB: bound by DRAM.
+// One pair of 1280x720, a launch at a time under ncu: rows 335 us (1.82 GB, 5.4 TB/s, integer ALU 78 %
+// busy), bottom to top 177 us (0.90 GB, 5.1 TB/s, 73 %), top to bottom with the WTA 312 us (1.90 GB,
+// 6.1 TB/s, 69 %): the last at 94 % of the measured copy bandwidth, the others between that (84 and 79 %)
+// and the integer ALU. The lane-per-disparity kernels they replace took 1582 us for the rows and 1961 us
+// for the columns (32-bit values, plain loads per step). With three pairs in flight a match takes 1.03 ms.
 #pragma once
 #include "sgm_async.cuh"
 #include "sgm_kernels4.cuh"

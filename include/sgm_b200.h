@@ -109,11 +109,14 @@ typedef struct sgm_tuning_t {
                            3 = cost-volume kernel + row_lanes lanes per scanline (u16x2 SIMD),
                            4 = one warp per scanline with cost chunks staged by bulk async copies
                            (path costs in 16-bit halves where exact, else in 32 bits): the shortest
-                           step chain, for one pair in flight (D <= 128 and tie rule 0, 1 or 4 at plain levels; any tie rule at the
-                           32-disparity pyramid levels; elsewhere the default);
+                           step chain, for one pair in flight (D <= 128 and tie rule 0, 1 or 4 at
+                           plain levels; any tie rule at the 32-disparity pyramid levels;
+                           elsewhere as 3 where that is exact, else 2);
                            0 (default) = 3 where it is exact (see below), else 2; at D = 256 with
                            every other member 0 too, rows and columns as in variant 4 (P1 <= 127,
-                           P1 <= P2 <= 16383 and tie rule 0 or 4, else 2 / 1) */
+                           P1 <= P2 <= 16383, tie rule 0 or 4, at most 65535 rows; else 2 / 1).
+                           A matcher left at the defaults that takes variant 4 also runs its views, or
+                           the next level's census, beside other work; one set to it by hand does not */
   int32_t rows_per_cta; /* scanlines per CTA of the horizontal scans: 0 (default), 1, 2 or 4 */
   int32_t col_kernel;   /* vertical scans + WTA: 1 = one warp per column, plain loads, 2 = the same with
                            an 8-row prefetch ring, 3 = col_lanes lanes per column (u16x2 SIMD, WTA in
